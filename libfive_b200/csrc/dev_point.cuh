@@ -107,7 +107,8 @@ __device__ __forceinline__ D4 d4_scale(float v, const D4& a, float f)
     return {v, __fmul_rn(a.dx, f), __fmul_rn(a.dy, f), __fmul_rn(a.dz, f)};
 }
 
-static __device__ __noinline__ D4 dv_deriv_all(uint8_t o, const D4& a, const D4& b,
+// By value: references would send every operand through local memory.
+static __device__ __noinline__ D4 dv_deriv_all(uint8_t o, const D4 a, const D4 b,
                                                bool clear_vars)
 {
     const float av = a.v, bv = b.v;
