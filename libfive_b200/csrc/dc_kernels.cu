@@ -190,7 +190,10 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane)
 /// are still to be read).  On straight-line code this uses as many registers
 /// as values are live at once, which is at most the unpruned tape's count;
 /// the leaf kernel then fits the register file of most leaf tapes in shared
-/// memory.  Values are unchanged: only storage moves.
+/// memory.  A copy (a decided min / max) whose source is not read again is
+/// dropped: its result takes over the source's register.  Union-heavy models
+/// leave one copy per decided level of their tree, a fifth to a third of a
+/// deep tape.  Values are unchanged: only storage moves.
 static __device__ __noinline__ TapeRef renumber_tape(uint2* raw_t, TapeRef tr,
                                                      uint8_t* lastuse,
                                                      uint16_t* regmap,
@@ -224,13 +227,17 @@ static __device__ __noinline__ TapeRef renumber_tape(uint2* raw_t, TapeRef tr,
     if (kMaxTapeRegs % 32) mask[kWords - 1] = (1u << (kMaxTapeRegs % 32)) - 1;
     mask[0] &= ~xyz_live;
     for (uint32_t r = 0; r < 3; ++r) regmap[r] = static_cast<uint16_t>(r);
-    uint32_t hi = 3;
+    uint32_t hi = 3, kept = 0;
     for (uint32_t c = 0; c < tr.len; ++c) {
         uint2 raw = raw_t[c];
         const uint32_t o = raw.x >> 16, kinds = (raw.x >> 8) & 0xff;
         const bool binary = dev_is_binary(raw.x & 0xff);
         uint32_t a = raw.y & 0xffff, b = raw.y >> 16;
         const uint8_t f = lastuse[c];
+        if ((raw.x & 0xff) == OP_COPY && (f & 1)) {
+            regmap[o] = regmap[a];
+            continue;
+        }
         if ((kinds & 3) == OPND_REG) a = regmap[a];
         if (binary && ((kinds >> 2) & 3) == OPND_REG) b = regmap[b];
         if (f & 1) mask[a >> 5] |= 1u << (a & 31);
@@ -251,10 +258,10 @@ static __device__ __noinline__ TapeRef renumber_tape(uint2* raw_t, TapeRef tr,
         hi = max(hi, r + 1);
         raw.x = (raw.x & 0xffffu) | (r << 16);
         raw.y = a | (b << 16);
-        raw_t[c] = raw;
+        raw_t[kept++] = raw;
     }
     const uint32_t root = rk == OPND_REG ? regmap[rr] : rr;
-    return {tr.off, tr.len, hi, root | (rk << 16)};
+    return {tr.off, kept, hi, root | (rk << 16)};
 }
 
 __global__ void __launch_bounds__(256)
@@ -522,7 +529,8 @@ k_interval_wide(WideArgs A, int d)
                     out_t = renumber_tape(buf, out_t, SM->live, SM->regmap, SM->mask, A.status);
                 }
                 __syncwarp();
-                for (uint32_t k = lane; k < emit; k += 32) dst[k] = buf[k];
+                out_t.len = __shfl_sync(full, out_t.len, 0);
+                for (uint32_t k = lane; k < out_t.len; k += 32) dst[k] = buf[k];
                 out_t.nregs = __shfl_sync(full, out_t.nregs, 0);
                 out_t.root = __shfl_sync(full, out_t.root, 0);
             }
@@ -965,22 +973,42 @@ k_interval_group(GroupArgs A, int d)
 
 
 struct EdgeSlot {
-    double t0[3], t1[3];   // current search bracket: inside, outside
-    float g0[4], g1[4];    // gradient + value at t0 / t1
-    uint8_t amb[2];        // tied min/max at t0 / t1
+    float g0[4], g1[4];    // gradient + value at the bracket's ends
+    uint8_t amb[2];        // tied min/max there
 };
 
-/// Per-warp state kept in shared memory (small: occupancy is set by it).
-struct LeafWarpShared {
-    int8_t slot_of[54];    // lattice edge -> slot, -1 if not crossing
-    uint8_t st[27];        // corner states (CELL_EMPTY / CELL_FILLED)
-    uint8_t nslots;
-    int32_t rec[8];
+/// A lattice edge's search bracket: inside end (x, y, z), outside end.
+struct EdgeBracket {
+    double t[6];
 };
 
-/// Per-warp state kept in global memory (L1-cached): edge brackets, the
-/// gradients at their final ends and the feature evaluator's scratch, one
-/// slice per resident warp.
+/// Zero-valued samples of a group's edge search that its QEF pass checks.
+constexpr uint32_t kLeafZeros = 48;
+
+constexpr uint32_t kLeafSteps = 56;   // steps of a tape in shared memory at a time
+constexpr uint32_t kLeafChunk = 4;    // groups taken at a time, with 16 or more a warp
+
+/// Per-warp state of the corner and edge-search kernel, in shared memory
+/// (24 warps an SM beside register files of kLeafSmemRegsMany registers).
+struct __align__(16) LeafWarpShared {
+    union {
+        ValOp vops[kLeafSteps];    // the tape's steps (short tapes: once a group)
+        LeafOp dops[kLeafOps];     // the derivative interpreter's clauses
+    };
+    EdgeBracket br[54];
+    double lats[kLeafChunk][3][3]; // lattice coordinates along each axis, by group
+    union {
+        float zpt[kLeafZeros][3];  // samples with a zero value, to be checked
+        uint8_t zlist[128];        // CAREFUL: their slots, to be settled here
+    };
+    uint32_t term[5];              // samples that are outside, by slot (one word more)
+    uint32_t zero[4];              // samples with a zero value
+    int8_t slot_of[54];            // lattice edge -> slot, -1 if not crossing
+};
+
+/// Per-warp state kept in global memory (L1-cached): the gradients at the
+/// edges' final bracket ends and the feature evaluator's scratch, one slice
+/// per resident warp.
 struct LeafWarpScratch {
     FeatureScratch fs;
     EdgeSlot e[54];
@@ -989,7 +1017,7 @@ struct LeafWarpScratch {
 /// A crossing lattice edge's QEF, handed from the leaf kernel to the rank
 /// and vertex kernels.
 struct EdgeRec {
-    double t0[3], t1[3];   // final search bracket: inside end, outside end
+    double t[6];   // final search bracket: inside end, outside end
     Qef q;
     uint8_t exists;
     uint8_t rank;
@@ -999,7 +1027,9 @@ struct EdgeRec {
 /// which (-1: none).
 struct GroupEdges {
     uint32_t base;          // 0xffffffff: the records did not fit
+    uint32_t zbase;         // its zero-valued samples in LeafArgs::zeros
     uint8_t n_edges;
+    uint8_t n_zeros;
     int8_t slot_of[54];
 };
 
@@ -1051,22 +1081,17 @@ __device__ __forceinline__ float4 dv_value4f(uint8_t o, const float4& a, const f
 }
 
 /// Values of the tape at four points per lane (point k of this lane in
-/// component k), streaming the tape's clauses (one clause fetched ahead) with
-/// the register file as one float4 per register and lane.  With ties
-/// (a run-time flag, so that one copy of the loop serves corners and edge
-/// search), bit k of *amb reports a min / max with equal arguments at point
-/// k (ArrayEvaluator::getAmbiguous, eval_array.cpp:197-217).
-template <bool S>
+/// component k) for tapes with more registers than the shared-memory file
+/// holds: the clauses are streamed (one fetched ahead), the register file R
+/// (x, y, z in its first three) is in global memory.  With ties, bit k of *amb reports a min / max with
+/// equal arguments at point k (ArrayEvaluator::getAmbiguous,
+/// eval_array.cpp:197-217).
 static __device__ __noinline__ float4 warp_value4(const float* __restrict__ cpool,
                                                   uint32_t root_kind, uint32_t root,
                                                   const RegClause* __restrict__ cl, uint32_t len,
-                                                  uint32_t soff, float* Rg, int lane, float4 x,
-                                                  float4 y, float4 z, bool ties, uint32_t* amb)
+                                                  float* Rg, int lane, bool ties, uint32_t* amb)
 {
-    float4* R = regfile4<S>(soff, Rg) + lane;
-    R[0] = x;
-    R[32] = y;
-    R[64] = z;
+    float4* R = reinterpret_cast<float4*>(Rg) + lane;
     uint32_t t = 0;
     uint2 next = len ? __ldg(reinterpret_cast<const uint2*>(cl)) : make_uint2(0, 0);
 #pragma unroll 1
@@ -1136,8 +1161,16 @@ static __device__ __noinline__ D4 leaf_deriv(const float* __restrict__ cpool, ui
     return {__ldg(cpool + root), 0.0f, 0.0f, 0.0f};
 }
 
-constexpr size_t kLeafSmallBytes = (sizeof(LeafWarpShared) + 15) / 16 * 16;
-constexpr uint32_t kLeafSmemRegs = 16;   // shared-memory register file per warp
+// Registers of the shared-memory register file per warp.  k_leaf_groups:
+// 8 when the groups fill the GPU (9.5 KB a warp, 24 warps an SM; 99 % of the
+// leaf tapes of CSG models use at most 8 registers, the others run from
+// global memory), 16 when all its warps fit beside each other anyway (at
+// most kLeafFewGroups groups); k_leaf_qef: 16.
+constexpr uint32_t kLeafSmemRegs = 16;
+constexpr uint32_t kLeafSmemRegsMany = 8;
+constexpr uint32_t kLeafFewGroups = 148 * 16;
+constexpr int kLeafWarps = 8, kLeafBlocks = 3;   // warps per block, blocks per SM
+static_assert(kLeafSmemRegs <= kValMaxRegs, "register offsets of a step are 16 bits");
 
 struct LeafArgs {
     Octree o;
@@ -1153,7 +1186,6 @@ struct LeafArgs {
     uint32_t smem_regs;         // registers of the shared-memory register file
     uint32_t* next_group;       // work counter (zero at launch)
     const uint32_t* order;      // processing order of the groups (or null)
-    unsigned long long* prof;   // debug: 8 per group (cycles by section, feature calls, E)
     float* featws;              // per warp: n_regs x kRegBlock floats of feature lists
     EdgeRec* edges;             // crossing-edge QEFs of all groups
     unsigned long long* edge_top;
@@ -1161,400 +1193,519 @@ struct LeafArgs {
     GroupEdges* group_edges;    // one per group
     uint32_t* rec_group;        // per leaf record: group * 8 + cell
     uint32_t* next_group2;      // work counter of k_leaf_qef (zero at launch)
+    ValOp* vops;                // decoded steps of a tape, from its clause offset on
+    uint32_t* n_steps;          // by clause offset: steps of the tape there
+    uint32_t chunk;             // groups a warp of k_leaf_groups takes at a time
+    float* zeros;               // zero-valued samples to check: x, y, z
+    unsigned int* zero_top;
+    uint32_t zero_cap;
+    uint32_t* redo;             // groups to search again, carefully
+    uint32_t* n_redo;
+    uint32_t* next_redo;        // work counters of the two kernels of that
 };
 
-__global__ void __launch_bounds__(256, 3)
-k_leaf_groups(LeafArgs A, uint32_t n_groups)
+/// The value interpreter's steps (leaf_interp.cuh) of every tape that leaf
+/// groups use, decoded once a tape: groups whose parents decided nothing
+/// share theirs (six groups a tape on deep CSG meshes).  Steps go to
+/// A.vops from the tape's own clause offset on (there are never more steps
+/// than clauses), their number to A.n_steps, where the first group to come
+/// claims the tape.  A kernel of its own: decoding in k_leaf_groups cost
+/// 1,000 instructions a group and its code the instruction cache
+/// (2,000-primitive CSG at depth 8: 1.95 ms with it, 1.38 ms without).
+__global__ void __launch_bounds__(128)
+k_leaf_decode(const __grid_constant__ LeafArgs A, const TapeRef* tapes, uint32_t n, uint32_t per_warp)
+{
+    __shared__ uint2 raws[4][kValRaw];
+    const uint32_t lane = threadIdx.x & 31;
+    uint2* raw = raws[threadIdx.x >> 5];
+    const uint32_t i = (blockIdx.x * 4 + (threadIdx.x >> 5)) * per_warp + lane;
+    uint32_t off = 0, len = 0;
+    if (lane < per_warp && i < n) {
+        const TapeRef t = tapes[i];
+        if (t.nregs <= A.smem_regs && t.len && A.n_steps[t.off] == 0 &&
+            atomicCAS(A.n_steps + t.off, 0u, 0xffffffffu) == 0) {
+            off = t.off;
+            len = t.len;
+        }
+    }
+    uint32_t todo = __ballot_sync(0xffffffffu, len != 0);
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t o = __shfl_sync(0xffffffffu, off, src);
+        const uint32_t l = __shfl_sync(0xffffffffu, len, src);
+        uint32_t steps = 0;
+        for (uint32_t c0 = 0; c0 < l; c0 += kLeafOps) {
+            steps += val_decode(A.vops + o + steps, raw, A.arena + o, l, c0, A.bt.cpool, lane);
+        }
+        if (lane == 0) A.n_steps[o] = steps;
+    }
+}
+
+/// FeatureEvaluator::isInside at one point (all lanes the same), out of line
+/// with its own contexts so that the leaf kernel's hot state stays in
+/// registers.
+static __device__ __noinline__ bool leaf_is_inside(const LeafArgs& A, TapeRef tr, uint32_t slice,
+                                                   float x, float y, float z, int lane)
+{
+    const FeatCtx fc{A.featws + static_cast<size_t>(slice) * A.bt.n_regs * kRegBlock,
+                     &A.scratch[slice].fs, A.status};
+    return dev_is_inside(fc, with_tape(A.bt, tr), A.arena + tr.off, tr.len, x, y, z, lane);
+}
+
+/// DCTree::evalLeaf's corners, classification and edge search
+/// (dc_tree.inl:156-410), one warp per sibling group.  SINGLE: the root cell
+/// is the only leaf (a 2 x 2 x 2 lattice instead of 3 x 3 x 3).
+///
+/// A sample whose value is exactly zero is inside or not by its gradient
+/// (FeatureEvaluator::isInside): for a point without tied min/max "gradient
+/// is non-zero" (one feature), otherwise the full feature search.  Nearly
+/// all are inside, and nearly every group has some in its last rounds.  So
+/// the search takes them for inside and writes them down, and k_leaf_qef,
+/// which evaluates gradients in any case and has lanes free, checks them; a
+/// group with a sample that is not inside (or more of them than there is
+/// room for) is listed in LeafArgs::redo and searched again by the CAREFUL
+/// form, which settles each zero where it meets it.  Evaluating gradients
+/// here instead took 2,500 of 10,000 instructions a group and, because the
+/// two interpreters' code then alternates, 37 % of the time (64-sphere
+/// union at depth 8: 1.71 ms against 1.08 ms).
+template <bool SINGLE, bool CAREFUL>
+__global__ void __launch_bounds__(32 * kLeafWarps, kLeafBlocks)
+k_leaf_groups(const __grid_constant__ LeafArgs A, uint32_t n_groups)
 {
     extern __shared__ __align__(16) unsigned char lsmem[];
-    // The edge search's sample fractions j / 15, divided once per block
-    // (the same correctly rounded quotients as dividing at every sample).
-    __shared__ double frac_tab[16];
-    if (threadIdx.x < 16) frac_tab[threadIdx.x] = threadIdx.x / (16 - 1.0);
+    constexpr int n = SINGLE ? 2 : 3;        // lattice points per axis
+    constexpr int seg = n - 1;
+    constexpr int ncell = SINGLE ? 1 : 8;
+    constexpr int npts = n * n * n;
+    constexpr int n_lat_edges = 3 * seg * n * n;
+    constexpr bool REDO = CAREFUL && !SINGLE;   // groups of the redo list
+    // The edge search's sample fractions j / 15 and 1 - j / 15, computed
+    // once per block (the same correctly rounded values as at every sample).
+    __shared__ double2 frac_tab[16];
+    if (threadIdx.x < 16) {
+        const double frac = threadIdx.x / (16 - 1.0);
+        frac_tab[threadIdx.x] = make_double2(frac, 1 - frac);
+    }
     __syncthreads();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
+    const unsigned full = 0xffffffffu;
     LeafWarpShared* S = reinterpret_cast<LeafWarpShared*>(lsmem) + warp;
-    // Register file of the tape interpreters (n_regs x 4 x 32 floats): in
-    // shared memory when the group's tape uses
-    // at most A.smem_regs registers (leaf tapes are renumbered compactly, so
-    // nearly all do), else in a per-warp slice of global memory.
-    float* Rs = reinterpret_cast<float*>(lsmem + kLeafSmallBytes * wpb) +
-                static_cast<size_t>(warp) * A.smem_regs * 128;
-    float* Rgl = A.rd + (static_cast<size_t>(blockIdx.x) * wpb + warp) * A.bt.n_regs * 128;
-    // Decoded clauses of the group's tape (leaf_interp.cuh), after the
-    // register files.
-    const uint32_t ops_off = static_cast<uint32_t>(kLeafSmallBytes * wpb +
-                                                   static_cast<size_t>(wpb) * A.smem_regs * 128 * 4 +
-                                                   static_cast<size_t>(warp) * kLeafOps * sizeof(LeafOp));
-    LeafWarpScratch* W = A.scratch + static_cast<size_t>(blockIdx.x) * wpb + warp;
-    uint64_t my_evals = 0, my_devals = 0;
-    // Persistent warps take the next group from a shared counter (group
-    // costs vary by orders of magnitude with the tape length).
-    while (true) {
-    uint32_t g = 0;
-    if (lane == 0) g = atomicAdd(A.next_group, 1u);
-    g = __shfl_sync(0xffffffffu, g, 0);
-    if (g >= n_groups) break;
-    if (A.order) g = A.order[g];
+    const uint32_t rsoff = static_cast<uint32_t>(sizeof(LeafWarpShared) * wpb +
+                                                 size_t{kValRegBytes} * A.smem_regs * warp);
+    const uint32_t ops_off = static_cast<uint32_t>(reinterpret_cast<unsigned char*>(S->dops) - lsmem);
+    unsigned char* Rl = lsmem + rsoff + 16 * lane;
+    const uint32_t slice = blockIdx.x * wpb + warp;   // of the per-warp global scratch
+    float* Rgl = A.rd + static_cast<size_t>(slice) * A.bt.n_regs * 128;
     const Octree& o = A.o;
     const int Ld = o.levels;
-    const bool single = (Ld == 0);       // the root itself is the only leaf
-    const int n = single ? 2 : 3;        // lattice points per axis
-    const int ncell = single ? 1 : 8;
-
-    // Lattice coordinates along each axis (double), from the parent region
-    // split at its centre exactly like Region::subdivide.
-    double lat[3][3];
-    TapeRef tr;
-    uint64_t base_coords;
-    if (single) {
-        for (int a = 0; a < 3; ++a) {
-            lat[a][0] = o.lo[a];
-            lat[a][1] = o.hi[a];
-        }
-        tr = root_tape_ref(A.bt);
-        base_coords = 0;
-    } else {
-        const LevelView& lv = o.lv[Ld];
-        const uint32_t parent = lv.group_parent[g];
-        const uint64_t pc = o.lv[Ld - 1].coords[parent];
-        double plo[3], phi[3];
-        cell_bounds(o, Ld - 1, pc, plo, phi);
-        for (int a = 0; a < 3; ++a) {
-            lat[a][0] = plo[a];
-            lat[a][1] = (plo[a] + phi[a]) / 2;
-            lat[a][2] = phi[a];
-        }
-        tr = lv.group_tape[g];
-        base_coords = pc;
-    }
-    const RegClause* cl = A.arena + tr.off;
-    const long long t_group = clock64();
-    unsigned long long feat_cycles = 0, feat_calls = 0;
-    const DevTape tb = with_tape(A.bt, tr);
-    const bool rs = tb.n_regs <= A.smem_regs;
-    float* R = rs ? Rs : Rgl;
-    const uint32_t rsoff = static_cast<uint32_t>(reinterpret_cast<unsigned char*>(Rs) - lsmem);
-#define RF_CALL(fn, ...) (rs ? fn<true>(__VA_ARGS__) : fn<false>(__VA_ARGS__))
-#define RF_VALUE4(...) (rs ? warp_value4<true>(__VA_ARGS__) : warp_value4<false>(__VA_ARGS__))
-    // Tapes that fit the buffer are decoded once for the whole group.
-    __syncwarp();
-    const FeatCtx fc{A.featws + (static_cast<size_t>(blockIdx.x) * wpb + warp) *
-                                    A.bt.n_regs * kRegBlock,
-                     &W->fs, A.status};
-
-    // --- corners (dc_tree.inl:156-239) ---------------------------------
-    const int npts = n * n * n;
-    float cv = 0.0f;
-    bool camb = false;
-    float px = 0, py = 0, pz = 0;
-    if (lane < npts) {
-        const int ia = lane % n, ib = (lane / n) % n, ic = lane / (n * n);
-        px = static_cast<float>(lat[0][ia]);
-        py = static_cast<float>(lat[1][ib]);
-        pz = static_cast<float>(lat[2][ic]);
+    // Persistent warps take the next groups from a shared counter (group
+    // costs vary by orders of magnitude with the tape length), a few at a
+    // time, so that the loads that lead to a group's tape and region overlap
+    // for all of them: one group a lane.
+    const uint32_t n_todo = REDO ? min(*A.n_redo, n_groups) : n_groups;
+    while (true) {
+    uint32_t g0 = 0;
+    if (lane == 0) g0 = atomicAdd(REDO ? A.next_redo : A.next_group, A.chunk);
+    g0 = __shfl_sync(full, g0, 0);
+    if (g0 >= n_todo) break;
+    const uint32_t n_here = min(A.chunk, n_todo - g0);
+    uint32_t lane_g = 0, lane_steps = 0;
+    TapeRef lane_tr{};
+    unsigned long long lane_pc = 0;
+    if (lane < n_here) {
+        lane_g = REDO ? A.redo[g0 + lane] : A.order ? A.order[g0 + lane] : g0 + lane;
+        lane_tr = SINGLE ? root_tape_ref(A.bt) : o.lv[Ld].group_tape[lane_g];
+        if (!SINGLE) lane_pc = o.lv[Ld - 1].coords[o.lv[Ld].group_parent[lane_g]];
+        if (lane_tr.len && lane_tr.nregs <= A.smem_regs) lane_steps = A.n_steps[lane_tr.off];
     }
     {
-        uint32_t amb4 = 0;
-        const float4 v4 = RF_VALUE4(tb.cpool, tb.root_kind, tb.root, cl, tr.len, rsoff, R,
-                                    lane, splat4(px), splat4(py), splat4(pz), true, &amb4);
-        cv = v4.x;
-        camb = (amb4 & 1) != 0;
-        const uint32_t act = __ballot_sync(0xffffffffu, lane < npts);
-        if (lane == 0) my_evals += static_cast<uint64_t>(__popc(act)) * tr.len;
-    }
-    uint8_t cst = CELL_EMPTY;
-    bool need_d = false, need_f = false;
-    if (lane < npts) {
-        if (cv > 0 || cv != cv) cst = CELL_EMPTY;
-        else if (cv < 0) cst = CELL_FILLED;
-        else if (!camb) need_d = true;
-        else need_f = true;
-    }
-    if (__any_sync(0xffffffffu, need_d || need_f)) {
-        bool amb = false, plain = false;
-        const D4 d = RF_CALL(leaf_deriv, tb.cpool, tb.root_kind, tb.root, tb.n_regs, cl,
-                             tr.len, rsoff, R, ops_off, lane, px, py, pz, &amb, &plain, false);
-        const uint32_t act = __ballot_sync(0xffffffffu, need_d || need_f);
-        if (lane == 0) my_devals += static_cast<uint64_t>(__popc(act)) * tr.len;
-        if (need_d) {
-            cst = (d.dx != 0 || d.dy != 0 || d.dz != 0) ? CELL_FILLED : CELL_EMPTY;
-        }
-        if (need_f && plain) {
-            // FeatureEvaluator::isInside with one feature at a zero value.
-            const float g[3] = {d.dx, d.dy, d.dz};
-            cst = sqrtf(fdot(g, g)) > 0 ? CELL_FILLED : CELL_EMPTY;
-            need_f = false;
-        }
-    }
-    {
-        uint32_t pending = __ballot_sync(0xffffffffu, need_f);
-        while (pending) {
-            const int src = __ffs(pending) - 1;
-            pending &= pending - 1;
-            const float qx = __shfl_sync(0xffffffffu, px, src);
-            const float qy = __shfl_sync(0xffffffffu, py, src);
-            const float qz = __shfl_sync(0xffffffffu, pz, src);
-            const long long t0 = clock64();
-            const bool inside = dev_is_inside(fc, tb, cl, tr.len, qx, qy, qz, lane);
-            feat_cycles += clock64() - t0;
-            ++feat_calls;
-            if (lane == src) cst = inside ? CELL_FILLED : CELL_EMPTY;
-        }
-    }
-    if (lane < npts) S->st[lane] = cst;
-    __syncwarp();
-
-    // --- cell classification --------------------------------------------
-    auto lat_pt = [&](int cell, int corner) {
-        const int cx = cell & 1, cy = (cell >> 1) & 1, cz = (cell >> 2) & 1;
-        return (cx + (corner & 1)) + n * ((cy + ((corner >> 1) & 1)) +
-                                          n * (cz + ((corner >> 2) & 1)));
-    };
-    const LevelView& lvL = o.lv[Ld];
-    if (lane < ncell) {
-        uint8_t mask = 0;
-        for (int k = 0; k < 8; ++k) {
-            mask |= (S->st[lat_pt(lane, k)] == CELL_FILLED ? 1 : 0) << k;
-        }
-        const uint32_t ci = single ? 0 : (g * 8 + lane);
-        int32_t rec = -1;
-        uint8_t type = mask == 0 ? CELL_EMPTY : mask == 0xff ? CELL_FILLED : CELL_LEAF;
-        if (type == CELL_LEAF) {
-            const uint32_t r = atomicAdd(A.rec_top, 1u);
-            if (r >= A.rec_cap) {
-                atomicOr(A.status, ST_RECORD_OVERFLOW);
+        // Lattice coordinates along each axis (double), from the parent
+        // region split at its centre exactly like Region::subdivide: lane 3
+        // i + a computes group i's axis a.
+        const int i = min(lane / 3, static_cast<int>(kLeafChunk) - 1), a = lane % 3;
+        const uint64_t pc = __shfl_sync(full, lane_pc, i);
+        if (lane < 3 * static_cast<int>(kLeafChunk)) {
+            double l = o.lo[a], h = o.hi[a];
+            double* lat = S->lats[i][a];
+            if (SINGLE) {
+                lat[0] = l;
+                lat[1] = h;
             } else {
-                rec = static_cast<int32_t>(r);
-                LeafRec& L = A.recs[r];
-                L.corner_mask = mask;
-                L.manifold = c_tab.manifold[mask];
-                L.vertex_count = c_tab.npatch[mask];
-                L.level = 0;
-                L.rank = 0;
+                const uint32_t idx = static_cast<uint32_t>(pc >> (21 * a)) & 0x1fffff;
+                for (int b = Ld - 2; b >= 0; --b) {
+                    const double m = (l + h) / 2;
+                    if ((idx >> b) & 1) l = m; else h = m;
+                }
+                lat[0] = l;
+                lat[1] = (l + h) / 2;
+                lat[n - 1] = h;
             }
         }
-        lvL.type[ci] = type;
-        lvL.rec[ci] = rec;
-        S->rec[lane] = rec;
     }
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t gi = 0; gi < n_here; ++gi) {
+    const uint32_t g = __shfl_sync(full, lane_g, gi);
+    const TapeRef tr{__shfl_sync(full, lane_tr.off, gi), __shfl_sync(full, lane_tr.len, gi),
+                     __shfl_sync(full, lane_tr.nregs, gi), __shfl_sync(full, lane_tr.root, gi)};
+    const uint32_t n_steps = __shfl_sync(full, lane_steps, gi);
+    if (REDO && A.group_edges[g].base == 0xffffffffu) continue;
+    const double (*lat)[3] = S->lats[gi];
+    const RegClause* cl = A.arena + tr.off;
+    const float* cpool = A.bt.cpool;
+    const uint32_t root_kind = tr.root >> 16, root = tr.root & 0xffff;
+    const bool rs = tr.nregs <= A.smem_regs;
+    // Tapes that fit the buffer are fetched once for the whole group (the
+    // derivative interpreter's clauses share it: CAREFUL fetches every pass).
+    auto fetch = [&](uint32_t s0) -> uint32_t {
+        const uint32_t m = min(kLeafSteps, n_steps - s0);
+        const uint4* src = reinterpret_cast<const uint4*>(A.vops + tr.off + s0);
+        __syncwarp();
+        for (uint32_t k = lane; k < 2 * m; k += 32) reinterpret_cast<uint4*>(S->vops)[k] = __ldg(src + k);
+        __syncwarp();
+        return m;
+    };
+    const bool once = !CAREFUL && n_steps <= kLeafSteps;
+    if (once) fetch(0);
 
-    const long long t_crossing = clock64();
-    // --- crossing lattice edges -----------------------------------------
-    const int seg = n - 1;
-    const int n_lat_edges = 3 * seg * n * n;
+    // Value and gradient at one point per lane, as leaf_deriv.
+    auto deriv = [&](float x, float y, float z, bool* amb, bool* plain) -> D4 {
+        return rs ? leaf_deriv<true>(cpool, root_kind, root, tr.nregs, cl, tr.len, rsoff,
+                                     Rgl, ops_off, lane, x, y, z, amb, plain, false)
+                  : leaf_deriv<false>(cpool, root_kind, root, tr.nregs, cl, tr.len, rsoff,
+                                      Rgl, ops_off, lane, x, y, z, amb, plain, false);
+    };
     auto lat_edge_ends = [&](int e, int& p0, int& p1) {
         const int ax = e / (seg * n * n);
         const int r = e % (seg * n * n);
         const int s = r % seg;
         const int u = (r / seg) % n;
         const int w = r / (seg * n);
-        int c0[3], c1[3];
-        if (ax == 0) { c0[0] = s; c0[1] = u; c0[2] = w; }
-        else if (ax == 1) { c0[1] = s; c0[0] = u; c0[2] = w; }
-        else { c0[2] = s; c0[0] = u; c0[1] = w; }
-        c1[0] = c0[0]; c1[1] = c0[1]; c1[2] = c0[2];
-        c1[ax] += 1;
-        p0 = c0[0] + n * (c0[1] + n * c0[2]);
-        p1 = c1[0] + n * (c1[1] + n * c1[2]);
+        const int step = ax == 0 ? 1 : ax == 1 ? n : n * n;
+        const int su = ax == 0 ? n : 1;
+        const int sw = ax == 2 ? n : n * n;
+        p0 = s * step + u * su + w * sw;
+        p1 = p0 + step;
     };
-    auto pt_pos = [&](int p, double out[3]) {
-        out[0] = lat[0][p % n];
-        out[1] = lat[1][(p / n) % n];
-        out[2] = lat[2][p / (n * n)];
+    // Sample j of an edge's bracket (dc_tree.inl:345-351).
+    auto sample = [&](int slot, int j) -> double3 {
+        const double2 f = frac_tab[j];
+        const EdgeBracket& es = S->br[slot];
+        return make_double3(es.t[0] * f.y + es.t[3] * f.x, es.t[1] * f.y + es.t[4] * f.x,
+                            es.t[2] * f.y + es.t[5] * f.x);
     };
-    if (lane == 0) S->nslots = 0;
-    __syncwarp();
-    for (int base = 0; base < n_lat_edges; base += 32) {
-        const int e = base + lane;
-        bool crossing = false;
-        int p0 = 0, p1 = 0;
-        if (e < n_lat_edges) {
-            lat_edge_ends(e, p0, p1);
-            crossing = S->st[p0] != S->st[p1];
-        }
-        const uint32_t m = __ballot_sync(0xffffffffu, crossing);
-        const int before = __popc(m & ((1u << lane) - 1));
-        const int first_slot = S->nslots;
-        if (e < n_lat_edges) {
-            S->slot_of[e] = crossing ? static_cast<int8_t>(first_slot + before) : -1;
-        }
-        if (crossing) {
-            EdgeSlot& es = W->e[first_slot + before];
-            const bool f0 = S->st[p0] == CELL_FILLED;
-            double a[3], b[3];
-            pt_pos(f0 ? p0 : p1, a);
-            pt_pos(f0 ? p1 : p0, b);
-            for (int k = 0; k < 3; ++k) { es.t0[k] = a[k]; es.t1[k] = b[k]; }
-        }
-        __syncwarp();
-        if (lane == 0) S->nslots = static_cast<uint8_t>(first_slot + __popc(m));
-        __syncwarp();
-    }
-    const int E = S->nslots;
+    // The loops below stay rolled where they can: 24 warps an SM in
+    // different places of this kernel miss the instruction cache otherwise
+    // (unrolled twice, the step loop ran 13 % fewer instructions in the same
+    // time, with three times the stalls on instruction fetch).
 
-    // --- edge search: 4 rounds of 16 points (dc_tree.inl:326-410) -------
-    // Each round samples an edge's bracket [t0, t1] at 16 evenly spaced
-    // points j = 0..15 and keeps [s(j-1), s(j)] around the first sample j >= 1
-    // that is outside; failing that, the last one, unless it is an inside
-    // zero.  s(0) = t0 is never tested, and s(15) = t1 is the previous
-    // round's outside end (round 1: the corner known to be outside), which is
-    // never an inside zero, so the outcome is "first outside j in 1..14,
-    // else 15": only 14 samples per edge are evaluated.  One pass holds nine
-    // edges (126 of the 4 x 32 sample slots): slot p = 32k + lane of
-    // sub-batch k is sample 1 + p % 14 of edge base + p / 14.  Most groups
-    // have nine crossing edges, one pass per round.
-    auto sample = [&](int slot, int j, double q[3]) {
-        const double frac = frac_tab[j];
-        const EdgeSlot& es = W->e[slot];
-        for (int k = 0; k < 3; ++k) q[k] = es.t0[k] * (1 - frac) + es.t1[k] * frac;
-    };
+    // --- passes: first the corners, then the edge search: 4 rounds of 16
+    // points (dc_tree.inl:326-410).  Each round samples an edge's bracket
+    // [t0, t1] at 16 evenly spaced points j = 0..15 and keeps
+    // [s(j-1), s(j)] around the first sample j >= 1 that is outside;
+    // failing that, the last one, unless it is an inside zero.  s(0) = t0
+    // is never tested, and s(15) = t1 is the previous round's outside end
+    // (round 1: the corner known to be outside), which is never an inside
+    // zero, so the outcome is "first outside j in 1..14, else 15": only 14
+    // samples per edge are evaluated.  One pass holds nine edges (126 of
+    // the 4 x 32 sample slots): slot p = 32k + lane of sub-batch k is
+    // sample 1 + p % 14 of edge base + p / 14.  Most groups have nine
+    // crossing edges, one pass per round.
     constexpr int kEdgesPerPass = 9, kSamples = 14;
-    for (int round = 0; round < 4; ++round) {
-        for (int base = 0; base < E; base += kEdgesPerPass) {
-            float qx[4] = {0, 0, 0, 0}, qy[4] = {0, 0, 0, 0}, qz[4] = {0, 0, 0, 0};
-            bool act[4];
-            int n_act = 0;
+    int E = 0, base = 0;
+    uint32_t n_zeros = 0;
+    for (int round = -1; round < 4;) {
+        // register file: x, y, z of the lane's four points
+        float* P = reinterpret_cast<float*>(rs ? Rl : reinterpret_cast<unsigned char*>(Rgl) + 16 * lane);
+        if (round < 0) {
+            const int q = lane < npts ? lane : 0;
+            const int c[3] = {q % n, (q / n) % n, q / (n * n)};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int p = 32 * k + lane;
-                const int slot = base + p / kSamples;
-                act[k] = p < kEdgesPerPass * kSamples && slot < E;
-                if (act[k]) {
-                    double q[3];
-                    sample(slot, 1 + p % kSamples, q);
-                    qx[k] = static_cast<float>(q[0]);
-                    qy[k] = static_cast<float>(q[1]);
-                    qz[k] = static_cast<float>(q[2]);
-                    ++n_act;
-                }
-            }
-            uint32_t unused = 0;
-            const float4 v4 = RF_VALUE4(tb.cpool, tb.root_kind, tb.root, cl, tr.len,
-                                        rsoff, R, lane,
-                                        make_float4(qx[0], qx[1], qx[2], qx[3]),
-                                        make_float4(qy[0], qy[1], qy[2], qy[3]),
-                                        make_float4(qz[0], qz[1], qz[2], qz[3]), false, &unused);
-            my_evals += static_cast<uint64_t>(__reduce_add_sync(0xffffffffu, n_act)) * tr.len;
-            const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
-            uint32_t term[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float v = vs[k];
-                // A sample exactly on the surface is resolved with
-                // FeatureEvaluator::isInside: for a point without tied
-                // min/max that is "gradient is non-zero" (one feature),
-                // otherwise the full feature search.
-                const bool zero = act[k] && v == 0;
-                bool inside = true;
-                if (__any_sync(0xffffffffu, zero)) {
-                    bool amb = false, plain = false;
-                    const D4 dg = RF_CALL(leaf_deriv, tb.cpool, tb.root_kind, tb.root,
-                                          tb.n_regs, cl, tr.len, rsoff, R, ops_off, lane,
-                                          qx[k], qy[k], qz[k], &amb, &plain, false);
-                    const uint32_t zact = __ballot_sync(0xffffffffu, zero);
-                    if (lane == 0) my_devals += static_cast<uint64_t>(__popc(zact)) * tr.len;
-                    amb = amb && !plain;   // a settled tie leaves one plain feature
-                    if (zero && !amb) {
-                        const float g[3] = {dg.dx, dg.dy, dg.dz};
-                        inside = sqrtf(fdot(g, g)) > 0;
-                    }
-                    uint32_t full = __ballot_sync(0xffffffffu, zero && amb);
-                    while (full) {
-                        const int src = __ffs(full) - 1;
-                        full &= full - 1;
-                        const float zx = __shfl_sync(0xffffffffu, qx[k], src);
-                        const float zy = __shfl_sync(0xffffffffu, qy[k], src);
-                        const float zz = __shfl_sync(0xffffffffu, qz[k], src);
-                        const long long t0 = clock64();
-                        const bool in = dev_is_inside(fc, tb, cl, tr.len, zx, zy, zz, lane);
-                        feat_cycles += clock64() - t0;
-                        ++feat_calls;
-                        if (lane == src) inside = in;
-                    }
-                }
-                term[k] = __ballot_sync(0xffffffffu, act[k] && (v > 0 || (v == 0 && !inside)));
-            }
-            // New brackets, one lane per edge, from the old ones.
-            if (lane < kEdgesPerPass && base + lane < E) {
-                const int p0 = kSamples * lane;
-                const int w0 = p0 >> 5, sh = p0 & 31;
-                uint32_t lo_w = 0, hi_w = 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (k == w0) lo_w = term[k];
-                    if (k == w0 + 1) hi_w = term[k];
-                }
-                const uint64_t bits = ((static_cast<uint64_t>(hi_w) << 32) | lo_w) >> sh;
-                const uint32_t t = static_cast<uint32_t>(bits) & ((1u << kSamples) - 1);
-                const int pick = t ? __ffs(t) : 15;   // sample index of the outside end
-                const int s_ = base + lane;
-                double nt0[3], nt1[3];
-                sample(s_, pick - 1, nt0);
-                sample(s_, pick, nt1);
-                EdgeSlot& es = W->e[s_];
-                for (int c = 0; c < 3; ++c) { es.t0[c] = nt0[c]; es.t1[c] = nt1[c]; }
-            }
-            __syncwarp();
-        }
-    }
-
-    const long long t_gradients = clock64();
-    const long long t_vertices = t_gradients;
-    // --- hand the final brackets to k_leaf_qef, the lattice edge map and
-    //     the records to the vertex kernel ---------------------------------
-    {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(A.edge_top, static_cast<unsigned long long>(E));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        const bool fits = base + E <= A.edge_cap;
-        GroupEdges& ge = A.group_edges[single ? 0 : g];
-        if (!fits) {
-            if (lane == 0) {
-                atomicOr(A.status, ST_EDGE_OVERFLOW);
-                ge.base = 0xffffffffu;
-                ge.n_edges = 0;
+            for (int a = 0; a < 3; ++a) {
+                reinterpret_cast<float4*>(P)[32 * a] = splat4(static_cast<float>(lat[a][c[a]]));
             }
         } else {
-            for (int s_ = lane; s_ < E; s_ += 32) {
-                EdgeRec& r = A.edges[base + s_];
-                for (int k = 0; k < 3; ++k) {
-                    r.t0[k] = W->e[s_].t0[k];
-                    r.t1[k] = W->e[s_].t1[k];
-                }
-            }
-            if (lane == 0) {
-                ge.base = static_cast<uint32_t>(base);
-                ge.n_edges = static_cast<uint8_t>(E);
-            }
-            for (int k = lane; k < n_lat_edges; k += 32) ge.slot_of[k] = S->slot_of[k];
-            if (lane < ncell && S->rec[lane] >= 0) {
-                A.rec_group[S->rec[lane]] = (single ? 0u : g * 8u) + static_cast<uint32_t>(lane);
+            // slots past the last sample repeat one, and are masked below
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+                const int p = 32 * k + lane;
+                const double3 q = sample(min(base + p / kSamples, E - 1), 1 + p % kSamples);
+                P[k] = static_cast<float>(q.x);
+                P[128 + k] = static_cast<float>(q.y);
+                P[256 + k] = static_cast<float>(q.z);
             }
         }
+        float4 v4;
+        uint32_t amb4 = 0;
+        if (rs) {
+            float last[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (uint32_t s0 = 0; s0 < n_steps; s0 += kLeafSteps) {
+                const uint32_t m = once ? n_steps : fetch(s0);
+                val_run(S->vops, m, Rl, round < 0, amb4, last);
+            }
+            v4 = root_kind == OPND_REG
+                     ? *reinterpret_cast<const float4*>(Rl + kValRegBytes * root)
+                     : splat4(__ldg(cpool + root));
+        } else {
+            v4 = warp_value4(cpool, root_kind, root, cl, tr.len, Rgl, lane, round < 0, &amb4);
+        }
+
+        if (round < 0) {
+            // --- corners (dc_tree.inl:156-239) -------------------------
+            const float cv = v4.x;
+            uint8_t cst = CELL_EMPTY;
+            bool need_d = false, need_f = false;
+            if (lane < npts) {
+                if (cv > 0 || cv != cv) cst = CELL_EMPTY;
+                else if (cv < 0) cst = CELL_FILLED;
+                else if (!(amb4 & 1)) need_d = true;
+                else need_f = true;
+            }
+            const uint32_t zeros = __ballot_sync(full, need_d || need_f);
+            if (zeros) {
+                bool amb = false, plain = false;
+                const int q = lane < npts ? lane : 0;
+                const float px = static_cast<float>(lat[0][q % n]);
+                const float py = static_cast<float>(lat[1][(q / n) % n]);
+                const float pz = static_cast<float>(lat[2][q / (n * n)]);
+                const D4 d = deriv(px, py, pz, &amb, &plain);
+                if (once) fetch(0);
+                if (lane == 0) atomicAdd(A.evals + 1, static_cast<unsigned long long>(__popc(zeros)) * tr.len);
+                if (need_d) {
+                    cst = (d.dx != 0 || d.dy != 0 || d.dz != 0) ? CELL_FILLED : CELL_EMPTY;
+                }
+                if (need_f && plain) {
+                    // FeatureEvaluator::isInside with one feature at a zero value.
+                    const float gr[3] = {d.dx, d.dy, d.dz};
+                    cst = sqrtf(fdot(gr, gr)) > 0 ? CELL_FILLED : CELL_EMPTY;
+                    need_f = false;
+                }
+                uint32_t pending = __ballot_sync(full, need_f);
+                while (pending) {
+                    const int src = __ffs(pending) - 1;
+                    pending &= pending - 1;
+                    const float fx = __shfl_sync(full, px, src);
+                    const float fy = __shfl_sync(full, py, src);
+                    const float fz = __shfl_sync(full, pz, src);
+                    const bool inside = leaf_is_inside(A, tr, slice, fx, fy, fz, lane);
+                    if (lane == src) cst = inside ? CELL_FILLED : CELL_EMPTY;
+                }
+            }
+            const uint32_t filled = __ballot_sync(full, lane < npts && cst == CELL_FILLED);
+
+            // --- cell classification -----------------------------------
+            const LevelView& lvL = o.lv[Ld];
+            if (!REDO && lane < ncell) {
+                const int cx = lane & 1, cy = (lane >> 1) & 1, cz = (lane >> 2) & 1;
+                uint32_t mask = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int p = (cx + (k & 1)) + n * ((cy + ((k >> 1) & 1)) +
+                                                        n * (cz + ((k >> 2) & 1)));
+                    mask |= ((filled >> p) & 1) << k;
+                }
+                const uint32_t ci = SINGLE ? 0 : (g * 8 + lane);
+                int32_t rec = -1;
+                const uint8_t type = mask == 0 ? CELL_EMPTY : mask == 0xff ? CELL_FILLED : CELL_LEAF;
+                if (type == CELL_LEAF) {
+                    const uint32_t r = atomicAdd(A.rec_top, 1u);
+                    if (r >= A.rec_cap) {
+                        atomicOr(A.status, ST_RECORD_OVERFLOW);
+                    } else {
+                        rec = static_cast<int32_t>(r);
+                        LeafRec& L = A.recs[r];
+                        L.corner_mask = static_cast<uint8_t>(mask);
+                        L.manifold = c_tab.manifold[mask];
+                        L.vertex_count = c_tab.npatch[mask];
+                        L.level = 0;
+                        L.rank = 0;
+                        A.rec_group[r] = (SINGLE ? 0u : g * 8u) + static_cast<uint32_t>(lane);
+                    }
+                }
+                lvL.type[ci] = type;
+                lvL.rec[ci] = rec;
+            }
+
+            // --- crossing lattice edges --------------------------------
+#pragma unroll 1
+            for (int e0 = 0; e0 < n_lat_edges; e0 += 32) {
+                const int e = e0 + lane;
+                bool crossing = false;
+                int p0 = 0, p1 = 0;
+                if (e < n_lat_edges) {
+                    lat_edge_ends(e, p0, p1);
+                    crossing = ((filled >> p0) ^ (filled >> p1)) & 1;
+                }
+                const uint32_t m = __ballot_sync(full, crossing);
+                const int slot = E + __popc(m & ((1u << lane) - 1));
+                if (e < n_lat_edges) S->slot_of[e] = crossing ? static_cast<int8_t>(slot) : -1;
+                if (crossing) {
+                    const bool f0 = (filled >> p0) & 1;
+                    const int in = f0 ? p0 : p1, out = f0 ? p1 : p0;
+                    EdgeBracket& es = S->br[slot];
+                    es.t[0] = lat[0][in % n];
+                    es.t[1] = lat[1][(in / n) % n];
+                    es.t[2] = lat[2][in / (n * n)];
+                    es.t[3] = lat[0][out % n];
+                    es.t[4] = lat[1][(out / n) % n];
+                    es.t[5] = lat[2][out / (n * n)];
+                }
+                E += __popc(m);
+            }
+            __syncwarp();
+            if (E == 0) break;
+            round = 0;
+            continue;
+        }
+
+        // --- one pass of the edge search -------------------------------
+        const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
+        const int n_act = kSamples * min(kEdgesPerPass, E - base);
+        uint32_t any_zero = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t act = n_act >= 32 * (k + 1) ? full
+                                 : n_act > 32 * k ? (1u << (n_act - 32 * k)) - 1 : 0u;
+            const uint32_t t = __ballot_sync(full, vs[k] > 0) & act;
+            const uint32_t z = __ballot_sync(full, vs[k] == 0) & act;
+            if (lane == k) {
+                S->term[k] = t;
+                S->zero[k] = z;
+            }
+            any_zero |= z;
+        }
+        __syncwarp();
+        // The 14 samples' bits of the pass's edge e.
+        auto edge_bits = [&](int e) -> uint32_t {
+            const int p0 = kSamples * e;
+            return __funnelshift_r(S->term[p0 >> 5], S->term[(p0 >> 5) + 1], p0 & 31) &
+                   ((1u << kSamples) - 1);
+        };
+        if (any_zero) {
+            // Zeros before the edge's first positive sample, gathered one
+            // per lane: CAREFUL settles them, otherwise they go on the list.
+            uint32_t nz = CAREFUL ? 0 : n_zeros;
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+                if (!S->zero[k]) continue;
+                const int p = 32 * k + lane;
+                const uint32_t t = edge_bits(p / kSamples);
+                const bool need = ((S->zero[k] >> lane) & 1) && (!t || p % kSamples < __ffs(t) - 1);
+                const uint32_t m = __ballot_sync(full, need);
+                const uint32_t at = nz + __popc(m & ((1u << lane) - 1));
+                if (need) {
+                    if (CAREFUL) {
+                        S->zlist[at] = static_cast<uint8_t>(p);
+                    } else if (at < kLeafZeros) {
+                        const double3 q = sample(base + p / kSamples, 1 + p % kSamples);
+                        S->zpt[at][0] = static_cast<float>(q.x);
+                        S->zpt[at][1] = static_cast<float>(q.y);
+                        S->zpt[at][2] = static_cast<float>(q.z);
+                    }
+                }
+                nz += __popc(m);
+            }
+            __syncwarp();
+            if (!CAREFUL) n_zeros = nz;
+            if (CAREFUL && nz && lane == 0) {
+                atomicAdd(A.evals + 1, static_cast<unsigned long long>(nz) * tr.len);
+            }
+            for (uint32_t i0 = 0; CAREFUL && i0 < nz; i0 += 32) {
+                const bool on = i0 + lane < nz;
+                const int p = S->zlist[on ? i0 + lane : 0];
+                const double3 q = sample(base + p / kSamples, 1 + p % kSamples);
+                const float zx = static_cast<float>(q.x);
+                const float zy = static_cast<float>(q.y);
+                const float zz = static_cast<float>(q.z);
+                bool amb = false, plain = false;
+                const D4 dg = deriv(zx, zy, zz, &amb, &plain);
+                amb = amb && !plain;   // a settled tie leaves one plain feature
+                const float gr[3] = {dg.dx, dg.dy, dg.dz};
+                bool inside = !on || amb || sqrtf(fdot(gr, gr)) > 0;
+                uint32_t pending = __ballot_sync(full, on && amb);
+                while (pending) {
+                    const int src = __ffs(pending) - 1;
+                    pending &= pending - 1;
+                    const float fx = __shfl_sync(full, zx, src);
+                    const float fy = __shfl_sync(full, zy, src);
+                    const float fz = __shfl_sync(full, zz, src);
+                    const bool in = leaf_is_inside(A, tr, slice, fx, fy, fz, lane);
+                    if (lane == src) inside = in;
+                }
+                if (!inside) atomicOr(&S->term[p >> 5], 1u << (p & 31));
+                __syncwarp();
+            }
+        }
+        // New brackets from the old ones: lanes 2 e and 2 e + 1 make edge e's
+        // inside and outside end.
+        const int e = min(min(lane >> 1, kEdgesPerPass - 1), E - 1 - base);
+        const uint32_t t = edge_bits(e);
+        const int pick = t ? __ffs(t) : 15;   // sample index of the outside end
+        const double3 q = sample(base + e, pick - 1 + (lane & 1));
+        __syncwarp();
+        if (e == lane >> 1) {
+            double* to = S->br[base + e].t + 3 * (lane & 1);
+            to[0] = q.x;
+            to[1] = q.y;
+            to[2] = q.z;
+        }
+        __syncwarp();
+        base += kEdgesPerPass;
+        if (base >= E) {
+            base = 0;
+            ++round;
+        }
     }
-    (void)base_coords;
-    if (A.prof && lane == 0) {
-        const long long t_end = clock64();
-        unsigned long long* P = A.prof + 8ull * g;
-        P[0] = t_end - t_group;
-        P[1] = feat_cycles;
-        P[2] = feat_calls;
-        P[3] = E;
-        P[4] = t_crossing - t_group;      // corners, classification
-        P[5] = t_gradients - t_crossing;  // crossing edges, edge search
-        P[6] = t_vertices - t_gradients;  // gradients, QEF pushes
-        P[7] = t_end - t_vertices;        // edge records
+
+    // --- hand the final brackets and the lattice edge map to k_leaf_qef and
+    //     the vertex kernel --------------------------------------------------
+    GroupEdges& ge = A.group_edges[SINGLE ? 0 : g];
+    unsigned long long first = 0;
+    if (REDO) {
+        first = ge.base;
+    } else {
+        if (lane == 0) first = atomicAdd(A.edge_top, static_cast<unsigned long long>(E));
+        first = __shfl_sync(full, first, 0);
+    }
+    if (first + E > A.edge_cap) {
+        if (lane == 0) {
+            atomicOr(A.status, ST_EDGE_OVERFLOW);
+            ge.base = 0xffffffffu;
+            ge.n_edges = 0;
+        }
+    } else {
+        for (int k = lane; k < 6 * E; k += 32) A.edges[first + k / 6].t[k % 6] = S->br[k / 6].t[k % 6];
+        uint32_t zbase = 0;
+        if (!CAREFUL && n_zeros) {
+            if (n_zeros <= kLeafZeros) {
+                if (lane == 0) zbase = atomicAdd(A.zero_top, n_zeros);
+                zbase = __shfl_sync(full, zbase, 0);
+            }
+            if (n_zeros > kLeafZeros || zbase > A.zero_cap || n_zeros > A.zero_cap - zbase) {
+                if (lane == 0) A.redo[atomicAdd(A.n_redo, 1u)] = g;
+                n_zeros = 0;
+            }
+            for (uint32_t k = lane; k < 3 * n_zeros; k += 32) {
+                A.zeros[size_t{3} * zbase + k] = S->zpt[k / 3][k % 3];
+            }
+        }
+        if (lane == 0) {
+            ge.base = static_cast<uint32_t>(first);
+            ge.n_edges = static_cast<uint8_t>(E);
+            ge.zbase = zbase;
+            ge.n_zeros = static_cast<uint8_t>(n_zeros);
+        }
+        for (int k = lane; k < n_lat_edges; k += 32) ge.slot_of[k] = S->slot_of[k];
+    }
+    if (lane == 0) {
+        atomicAdd(A.evals, static_cast<unsigned long long>(npts + 4 * kSamples * E) * tr.len);
+    }
+    __syncwarp();
     }
     }   // groups
-#undef RF_CALL
-#undef RF_VALUE4
-    if (lane == 0) {
-        atomicAdd(A.evals, static_cast<unsigned long long>(my_evals));
-        atomicAdd(A.evals + 1, static_cast<unsigned long long>(my_devals));
-    }
 }
 
 /// Gradients at the two ends of every crossing edge's final bracket and the
@@ -1564,6 +1715,9 @@ k_leaf_groups(LeafArgs A, uint32_t n_groups)
 /// gradient instead (eval_feature.cpp:125-169).  A launch of its own, so
 /// that the derivative interpreter does not share the instruction cache
 /// with the value interpreter of the edge search.
+/// The group's zero-valued samples are checked along with them (REDO: not,
+/// the groups of the redo list after their careful search).
+template <bool REDO>
 __global__ void __launch_bounds__(256, 3)
 k_leaf_qef(LeafArgs A, uint32_t n_groups)
 {
@@ -1571,11 +1725,9 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
-    float* Rs = reinterpret_cast<float*>(lsmem + kLeafSmallBytes * wpb) +
-                static_cast<size_t>(warp) * A.smem_regs * 128;
+    float* Rs = reinterpret_cast<float*>(lsmem) + static_cast<size_t>(warp) * A.smem_regs * 128;
     float* Rgl = A.rd + (static_cast<size_t>(blockIdx.x) * wpb + warp) * A.bt.n_regs * 128;
-    const uint32_t ops_off = static_cast<uint32_t>(kLeafSmallBytes * wpb +
-                                                   static_cast<size_t>(wpb) * A.smem_regs * 128 * 4 +
+    const uint32_t ops_off = static_cast<uint32_t>(static_cast<size_t>(wpb) * A.smem_regs * 128 * 4 +
                                                    static_cast<size_t>(warp) * kLeafOps * sizeof(LeafOp));
     LeafWarpScratch* W = A.scratch + static_cast<size_t>(blockIdx.x) * wpb + warp;
     const FeatCtx fc{A.featws + (static_cast<size_t>(blockIdx.x) * wpb + warp) *
@@ -1587,10 +1739,11 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
     const bool single = (Ld == 0);
     while (true) {
         uint32_t g = 0;
-        if (lane == 0) g = atomicAdd(A.next_group2, 1u);
+        if (lane == 0) g = atomicAdd(REDO ? A.next_redo + 1 : A.next_group2, 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
-        if (g >= n_groups) break;
-        if (A.order) g = A.order[g];
+        if (g >= (REDO ? min(*A.n_redo, n_groups) : n_groups)) break;
+        if (REDO) g = A.redo[g];
+        else if (A.order) g = A.order[g];
         const GroupEdges& ge = A.group_edges[single ? 0 : g];
         const uint32_t gbase = ge.base;
         const int E = ge.n_edges;
@@ -1607,26 +1760,39 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
                               tb.cpool, lane);
         }
         EdgeRec* er = A.edges + gbase;
-        for (int base = 0; base < 2 * E; base += 32) {
+        const float* zp = A.zeros + size_t{3} * ge.zbase;
+        const int n_pts = 2 * E + (REDO ? 0 : ge.n_zeros);
+        bool outside = false;   // a zero-valued sample that is not inside
+        for (int base = 0; base < n_pts; base += 32) {
             const int p = base + lane;
-            const bool active = p < 2 * E;
-            double q[3] = {0, 0, 0};
+            const bool active = p < 2 * E, check = !active && p < n_pts;
+            float q[3] = {0, 0, 0};
             if (active) {
                 const EdgeRec& e = er[p >> 1];
-                for (int k = 0; k < 3; ++k) q[k] = (p & 1) ? e.t1[k] : e.t0[k];
+                for (int k = 0; k < 3; ++k) q[k] = static_cast<float>(e.t[(p & 1) * 3 + k]);
+            } else if (check) {
+                for (int k = 0; k < 3; ++k) q[k] = zp[3 * (p - 2 * E) + k];
             }
             bool amb = false, plain = false;
             const D4 d = rs ? leaf_deriv<true>(tb.cpool, tb.root_kind, tb.root, tb.n_regs, cl,
-                                               tr.len, rsoff, R, ops_off, lane,
-                                               static_cast<float>(q[0]), static_cast<float>(q[1]),
-                                               static_cast<float>(q[2]), &amb, &plain, true)
+                                               tr.len, rsoff, R, ops_off, lane, q[0], q[1], q[2],
+                                               &amb, &plain, true)
                             : leaf_deriv<false>(tb.cpool, tb.root_kind, tb.root, tb.n_regs, cl,
-                                                tr.len, rsoff, R, ops_off, lane,
-                                                static_cast<float>(q[0]), static_cast<float>(q[1]),
-                                                static_cast<float>(q[2]), &amb, &plain, true);
-            const uint32_t gact = __ballot_sync(0xffffffffu, active);
-            if (lane == 0) my_devals += static_cast<uint64_t>(__popc(gact)) * tr.len;
+                                                tr.len, rsoff, R, ops_off, lane, q[0], q[1], q[2],
+                                                &amb, &plain, true);
+            if (lane == 0) my_devals += static_cast<uint64_t>(min(32, n_pts - base)) * tr.len;
             amb = amb && !plain;   // a settled tie leaves one plain feature
+            const float gr[3] = {d.dx, d.dy, d.dz};
+            outside |= check && !amb && !(sqrtf(fdot(gr, gr)) > 0);
+            uint32_t pending = __ballot_sync(0xffffffffu, check && amb);
+            while (pending) {
+                const int src = __ffs(pending) - 1;
+                pending &= pending - 1;
+                const float fx = __shfl_sync(0xffffffffu, q[0], src);
+                const float fy = __shfl_sync(0xffffffffu, q[1], src);
+                const float fz = __shfl_sync(0xffffffffu, q[2], src);
+                outside |= !dev_is_inside(fc, tb, cl, tr.len, fx, fy, fz, lane);
+            }
             if (active) {
                 EdgeSlot& es = W->e[p >> 1];
                 float* gg = (p & 1) ? es.g1 : es.g0;
@@ -1635,6 +1801,10 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
             }
         }
         __syncwarp();
+        if (!REDO && __any_sync(0xffffffffu, outside)) {
+            if (lane == 0) A.redo[atomicAdd(A.n_redo, 1u)] = g;
+            continue;
+        }
         const uint32_t any_amb = __ballot_sync(0xffffffffu, [&] {
             bool a = false;
             for (int s_ = lane; s_ < E; s_ += 32) a |= W->e[s_].amb[0] || W->e[s_].amb[1];
@@ -1648,7 +1818,7 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
                 qef_zero(qf);
                 for (int side = 0; side < 2; ++side) {
                     const float* gg = side ? es.g1 : es.g0;
-                    const double* pos = side ? r.t1 : r.t0;
+                    const double* pos = r.t + 3 * side;
                     const double gd[3] = {gg[0], gg[1], gg[2]};
                     qef_push(qf, pos, gd, static_cast<double>(gg[3]));
                 }
@@ -1668,7 +1838,7 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
                 EdgeRec& r = er[s_];
                 for (int side = 0; side < 2; ++side) {
                     const float* gg = side ? es.g1 : es.g0;
-                    const double* pos = side ? r.t1 : r.t0;
+                    const double* pos = r.t + 3 * side;
                     if (es.amb[side]) {
                         dev_push_features(fc, tb, cl, tr.len, pos, static_cast<double>(gg[3]),
                                           &r.q, &r.exists, lane);
@@ -2456,8 +2626,9 @@ enum BufKey {
     K_CUBTMP, K_TASK_A, K_TASK_B, K_TRIS, K_USED, K_VSCAN, K_VERTS, K_FEAT,
     K_LIST_A, K_LIST_B, K_WIDE_S, K_WIDE_SN, K_WIDE_P, K_WIDE_LIVE, K_WIDE_NEW,
     K_WIDE_ST2, K_WIDE_L1, K_WIDE_WL, K_LEAF_RD, K_ORDER_K0, K_ORDER_K1,
-    K_ORDER_V0, K_ORDER_V1, K_SORTTMP, K_PROF, K_GDEC, K_GLAST, K_FEATWS,
-    K_EDGES, K_GEDGES, K_RECGROUP, K_NREGS, K_STL, K_COORDS,
+    K_ORDER_V0, K_ORDER_V1, K_SORTTMP, K_GDEC, K_GLAST, K_FEATWS,
+    K_EDGES, K_GEDGES, K_RECGROUP, K_NREGS, K_STL, K_COORDS, K_ZEROS, K_REDO,
+    K_VOPS, K_NSTEPS, K_ROOTTAPE,
     K_LEVEL = 100,
 };
 
@@ -2932,6 +3103,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
     if (!gdec || !glast || !level_nregs) return LFB_E_CUDA;
     cudaMemsetAsync(level_nregs, 0, (kMaxLevels + 2) * sizeof(uint32_t), s);
     bool group_mode = false;
+    unsigned long long arena_used = bt.n;   // clauses in the arena
 
     for (int d = 0; d < L; ++d) {
         if (cancelled()) return LFB_E_CANCELLED;
@@ -3008,6 +3180,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             if (st & ST_REGS) {
                 return set_error(LFB_E_UNSUPPORTED, "tape register renumbering failed");
             }
+            arena_used = tops[0];
             if (!(st & (ST_ARENA_OVERFLOW | ST_LIST_OVERFLOW))) break;
             if (attempt == 3) return set_error(LFB_E_CAPACITY, "tape arena overflow");
             // The counters kept counting past the capacity: grow to what this
@@ -3090,11 +3263,10 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
     LeafRec* recs = ws.get<LeafRec>(K_RECS, rec_cap);
     if (!recs) return LFB_E_CUDA;
     if (n_leaf_groups) {
-        // Shared memory per warp: the small lattice state and a register
-        // file of smem_regs x 4 x 32 floats; groups whose tape needs more
-        // registers use global memory instead.
-        const int wpb = 8;
-        const uint32_t smem_regs = std::min<uint32_t>(bt.n_regs, kLeafSmemRegs);
+        // Warps per block: eight, fewer while that leaves SMs without a block.
+        const uint32_t sms = static_cast<uint32_t>(device_sm_count());
+        uint32_t wpb = kLeafWarps;
+        while (wpb > 1 && n_leaf_groups < sms * wpb) wpb /= 2;
         if (debug_levels() && L > 0) {
             std::vector<TapeRef> gt(n_leaf_groups);
             cudaMemcpyAsync(gt.data(), o.lv[L].group_tape, n_leaf_groups * sizeof(TapeRef),
@@ -3121,23 +3293,32 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             }
             std::fprintf(stderr, "\n");
         }
-        const size_t per_warp = kLeafSmallBytes + static_cast<size_t>(smem_regs) * 128 * 4 +
-                                kLeafOps * sizeof(LeafOp);
-        const size_t smem = per_warp * wpb;
-        if (smem > 220 * 1024) {
-            return set_error(LFB_E_UNSUPPORTED, "tape register file too large for the leaf kernel");
-        }
-        if (!raise_smem_limit(reinterpret_cast<const void*>(k_leaf_groups), smem)) {
+        // Shared memory: per warp its state and a register file of smem_regs
+        // float4s a lane; groups whose tape needs more registers use global
+        // memory instead.
+        const uint32_t group_regs = std::min<uint32_t>(
+            bt.n_regs, n_leaf_groups <= kLeafFewGroups ? kLeafSmemRegs : kLeafSmemRegsMany);
+        const uint32_t qef_regs = std::min<uint32_t>(bt.n_regs, kLeafSmemRegs);
+        const size_t group_bytes = (sizeof(LeafWarpShared) + size_t{512} * group_regs) * wpb;
+        const size_t qef_bytes = (sizeof(LeafOp) * kLeafOps + size_t{512} * qef_regs) * wpb;
+        auto* groups_kernel = L == 0 ? k_leaf_groups<true, true> : k_leaf_groups<false, false>;
+        auto* redo_kernel = k_leaf_groups<false, true>;
+        if (!raise_smem_limit(reinterpret_cast<const void*>(groups_kernel), group_bytes) ||
+            !raise_smem_limit(reinterpret_cast<const void*>(redo_kernel), group_bytes) ||
+            !raise_smem_limit(reinterpret_cast<const void*>(k_leaf_qef<false>), qef_bytes) ||
+            !raise_smem_limit(reinterpret_cast<const void*>(k_leaf_qef<true>), qef_bytes)) {
             return LFB_E_CUDA;
         }
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_leaf_groups, 32 * wpb, smem);
-        per_sm = std::max(per_sm, 1);
         const uint32_t want = (n_leaf_groups + wpb - 1) / wpb;
-        const uint32_t grid = std::min<uint32_t>(want, static_cast<uint32_t>(device_sm_count() * per_sm));
-        LeafWarpScratch* scratch = ws.get<LeafWarpScratch>(K_FEAT, static_cast<size_t>(grid) * wpb);
+        int per_sm = 0, qef_per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, groups_kernel, 32 * wpb, group_bytes);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qef_per_sm, k_leaf_qef<false>, 32 * wpb, qef_bytes);
+        const uint32_t grid = std::min<uint32_t>(want, sms * std::max(per_sm, 1));
+        const uint32_t qef_grid = std::min<uint32_t>(want, sms * std::max(qef_per_sm, 1));
+        const size_t slices = static_cast<size_t>(std::max(grid, qef_grid)) * wpb;
+        LeafWarpScratch* scratch = ws.get<LeafWarpScratch>(K_FEAT, slices);
         if (!scratch) return LFB_E_CUDA;
-        float* rd = ws.get<float>(K_LEAF_RD, static_cast<size_t>(grid) * wpb * bt.n_regs * 128);
+        float* rd = ws.get<float>(K_LEAF_RD, slices * bt.n_regs * 128);
         if (!rd) return LFB_E_CUDA;
         uint32_t* next_group = reinterpret_cast<uint32_t*>(counters + 7);
         cudaMemsetAsync(next_group, 0, sizeof(uint32_t), s);
@@ -3163,10 +3344,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             }
             order = v1;
         }
-        unsigned long long* prof = nullptr;
-        if (debug_levels()) prof = ws.get<unsigned long long>(K_PROF, 8ull * n_leaf_groups);
-        float* featws = ws.get<float>(K_FEATWS, static_cast<size_t>(grid) * wpb * bt.n_regs *
-                                                    kRegBlock);
+        float* featws = ws.get<float>(K_FEATWS, slices * bt.n_regs * kRegBlock);
         if (!featws) return LFB_E_CUDA;
         const uint64_t edge_cap64 = static_cast<uint64_t>(n_leaf_groups) * ws.edges_per_group +
                                     (small ? 0 : 1024);
@@ -3176,20 +3354,59 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         uint32_t* rec_group = ws.get<uint32_t>(K_RECGROUP, rec_cap);
         if (!edges || !gedges || !rec_group) return LFB_E_CUDA;
         cudaMemsetAsync(rec_group, 0xff, rec_cap * sizeof(uint32_t), s);
+        // Steps by clause offset, so room for as many as the arena has clauses.
+        ValOp* vops = ws.get<ValOp>(K_VOPS, arena_used);
+        uint32_t* n_steps = ws.get<uint32_t>(K_NSTEPS, arena_used);
+        if (!vops || !n_steps) return LFB_E_CUDA;
+        cudaMemsetAsync(n_steps, 0, arena_used * sizeof(uint32_t), s);
+        // Zero-valued samples: room for 32 a group on average (none with the
+        // small-capacity hook, so that every such group is searched again).
+        const uint32_t zero_cap = small ? 0u : static_cast<uint32_t>(std::min<uint64_t>(
+            static_cast<uint64_t>(n_leaf_groups) * 32 + 4096, 1u << 30));
+        float* zeros = ws.get<float>(K_ZEROS, size_t{3} * zero_cap);
+        uint32_t* redo = ws.get<uint32_t>(K_REDO, size_t{2} * n_leaf_groups + 4);
+        if (!zeros || !redo) return LFB_E_CUDA;
+        uint32_t* redo_counts = redo + 2 * static_cast<size_t>(n_leaf_groups);
+        cudaMemsetAsync(redo_counts, 0, 4 * sizeof(uint32_t), s);
         LeafArgs A{o, bt, arena, recs, rec_top, static_cast<uint32_t>(rec_cap), status,
-                   evals, scratch, rd, smem_regs, next_group, order, prof, featws,
+                   evals, scratch, rd, group_regs, next_group, order, featws,
                    edges, edge_top, edge_cap, gedges, rec_group,
-                   reinterpret_cast<uint32_t*>(counters + 9)};
-        k_leaf_groups<<<grid, 32 * wpb, smem, s>>>(A, n_leaf_groups);
-        if (!cuda_ok(cudaGetLastError(), "leaf kernel")) return LFB_E_CUDA;
-        if (!raise_smem_limit(reinterpret_cast<const void*>(k_leaf_qef), smem)) {
-            return LFB_E_CUDA;
+                   reinterpret_cast<uint32_t*>(counters + 9),
+                   vops, n_steps, n_leaf_groups >= kLeafChunk * 4 * grid * wpb ? kLeafChunk : 1u,
+                   zeros, redo_counts, zero_cap, redo, redo_counts + 1, redo_counts + 2};
+        const TapeRef* tapes = o.lv[L].group_tape;
+        if (L == 0) {
+            // the unpruned tape is the only one
+            TapeRef* t = reinterpret_cast<TapeRef*>(ws.get<uint4>(K_ROOTTAPE, 1));
+            const TapeRef root = root_tape_ref(bt);
+            if (!t || !cuda_ok(cudaMemcpyAsync(t, &root, sizeof(root), cudaMemcpyHostToDevice, s),
+                               "root tape")) {
+                return LFB_E_CUDA;
+            }
+            tapes = t;
         }
-        k_leaf_qef<<<grid, 32 * wpb, smem, s>>>(A, n_leaf_groups);
+        // groups per decoding warp: as few as fill the GPU
+        const uint32_t per_warp = std::min(32u, n_leaf_groups / (sms * 32) + 1);
+        k_leaf_decode<<<(n_leaf_groups + 4 * per_warp - 1) / (4 * per_warp), 128, 0, s>>>(
+            A, tapes, n_leaf_groups, per_warp);
         ++n_launch;
+        groups_kernel<<<grid, 32 * wpb, group_bytes, s>>>(A, n_leaf_groups);
+        if (!cuda_ok(cudaGetLastError(), "leaf kernel")) return LFB_E_CUDA;
+        A.smem_regs = qef_regs;
+        k_leaf_qef<false><<<qef_grid, 32 * wpb, qef_bytes, s>>>(A, n_leaf_groups);
+        ++n_launch;
+        if (L > 0) {
+            // the groups a check sent back (usually none)
+            const uint32_t few = std::min(grid, sms);
+            A.smem_regs = group_regs;
+            A.chunk = 1;
+            redo_kernel<<<few, 32 * wpb, group_bytes, s>>>(A, n_leaf_groups);
+            A.smem_regs = qef_regs;
+            k_leaf_qef<true><<<std::min(qef_grid, sms), 32 * wpb, qef_bytes, s>>>(A, n_leaf_groups);
+            n_launch += 2;
+        }
         if (!cuda_ok(cudaGetLastError(), "leaf QEF kernel")) return LFB_E_CUDA;
         // Edge ranks, then the records' vertices: one thread per edge / record.
-        const uint32_t sms = static_cast<uint32_t>(device_sm_count());
         k_edge_rank<<<std::min<uint32_t>(sms * 16, (edge_cap + 127) / 128), 128, 0, s>>>(
             edges, edge_top, edge_cap);
         k_leaf_vertices<<<std::min<uint32_t>(sms * 16, static_cast<uint32_t>((rec_cap + 127) / 128)),
@@ -3197,41 +3414,6 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
                                        gedges, n_leaf_groups, edges, edge_cap, L == 0 ? 1 : 0);
         n_launch += 2;
         if (!cuda_ok(cudaGetLastError(), "leaf vertex kernels")) return LFB_E_CUDA;
-        if (prof) {
-            std::vector<unsigned long long> pf(8ull * n_leaf_groups);
-            std::vector<TapeRef> gt(n_leaf_groups);
-            cudaMemcpyAsync(pf.data(), prof, pf.size() * 8, cudaMemcpyDeviceToHost, s);
-            if (L > 0) {
-                cudaMemcpyAsync(gt.data(), o.lv[L].group_tape, n_leaf_groups * sizeof(TapeRef),
-                                cudaMemcpyDeviceToHost, s);
-            }
-            cudaStreamSynchronize(s);
-            std::vector<uint32_t> idx(n_leaf_groups);
-            for (uint32_t k = 0; k < n_leaf_groups; ++k) idx[k] = k;
-            std::sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) { return pf[8 * a] > pf[8 * b]; });
-            unsigned long long sec[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (uint32_t k = 0; k < n_leaf_groups; ++k) {
-                for (int q = 0; q < 8; ++q) sec[q] += pf[8 * k + q];
-            }
-            {
-                std::map<uint32_t, uint64_t> eh;
-                for (uint32_t k = 0; k < n_leaf_groups; ++k) ++eh[static_cast<uint32_t>(pf[8 * k + 3])];
-                std::fprintf(stderr, "[lfb] crossing edges per group:");
-                for (const auto& h : eh) {
-                    std::fprintf(stderr, " %u:%llu", h.first, static_cast<unsigned long long>(h.second));
-                }
-                std::fprintf(stderr, "\n");
-            }
-            std::fprintf(stderr, "[lfb] leaf cycles total %llu: corners %llu, edge search %llu, "
-                         "gradients+QEF %llu, vertices %llu; features %llu in %llu calls\n",
-                         sec[0], sec[4], sec[5], sec[6], sec[7], sec[1], sec[2]);
-            for (uint32_t k = 0; k < std::min<uint32_t>(12, n_leaf_groups); ++k) {
-                const uint32_t gg = idx[k];
-                std::fprintf(stderr, "[lfb]   group %u: %llu cycles, features %llu cycles / %llu calls, E %llu, tape %u regs %u\n",
-                             gg, pf[8 * gg], pf[8 * gg + 1], pf[8 * gg + 2], pf[8 * gg + 3],
-                             L > 0 ? gt[gg].len : bt.n, L > 0 ? gt[gg].nregs : bt.n_regs);
-            }
-        }
         ++n_launch;
     }
     if (cancelled()) return LFB_E_CANCELLED;
