@@ -208,6 +208,10 @@ typedef struct lfb_mesh_stats {
     double ms_dual;
 } lfb_mesh_stats;
 
+/* memcpy over several host threads (additive: for bindings that copy a
+ * mesh's arrays into memory of their own). */
+void lfb_host_copy(void* dst, const void* src, uint64_t bytes);
+
 /* Number of kernels this library has launched since it was loaded. */
 uint64_t lfb_kernel_launches(void);
 

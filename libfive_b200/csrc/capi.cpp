@@ -859,6 +859,11 @@ int lfb_render_meshes(const lfb_tape* tapes, uint32_t n, const libfive_region3* 
     return rc;
 }
 
+void lfb_host_copy(void* dst, const void* src, uint64_t bytes)
+{
+    if (dst && src && bytes) lfb::host_copy(dst, src, bytes);
+}
+
 uint64_t lfb_kernel_launches(void) { return launches(); }
 
 int lfb_tree_slot_tape(libfive_tree t, uint32_t counts[8], int32_t* clauses,

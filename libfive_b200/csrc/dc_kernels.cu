@@ -2833,21 +2833,7 @@ bool download(Workspace& ws, void* dst, const void* src, size_t bytes, cudaStrea
         !cuda_ok(cudaStreamSynchronize(s), "download")) {
         return false;
     }
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t n_threads = std::min<size_t>(std::min<unsigned>(hw, 8u),
-                                              std::max<size_t>(1, bytes >> 22));
-    const size_t part = (bytes + n_threads - 1) / n_threads;
-    auto copy = [&](size_t t) {
-        const size_t lo = t * part, hi = std::min(bytes, lo + part);
-        if (lo < hi) {
-            std::memcpy(static_cast<char*>(dst) + lo, static_cast<const char*>(pinned) + lo,
-                        hi - lo);
-        }
-    };
-    std::vector<std::thread> pool;
-    for (size_t t = 1; t < n_threads; ++t) pool.emplace_back(copy, t);
-    copy(0);
-    for (auto& th : pool) th.join();
+    host_copy(dst, pinned, bytes);
     return true;
 }
 

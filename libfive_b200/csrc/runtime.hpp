@@ -27,6 +27,11 @@ bool require_device();
 /// Converts a CUDA status into an error record; returns true on success.
 bool cuda_ok(cudaError_t e, const char* what);
 
+/// memcpy between host blocks over a few threads: one thread moves (and
+/// first touches) a large mesh's arrays several times slower than the GPU
+/// makes them.
+void host_copy(void* dst, const void* src, size_t bytes);
+
 /// A tree flattened into both tape layouts, resident on the device.
 struct GpuTape {
     Tree tree;

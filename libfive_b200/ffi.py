@@ -180,6 +180,7 @@ SIGNATURES = [
                                          ctypes.POINTER(Region3), ctypes.POINTER(MeshSettings),
                                          ctypes.c_uint32, ctypes.POINTER(ctypes.POINTER(Mesh)),
                                          ctypes.POINTER(MeshStats)]),
+    ("lfb_host_copy", None, [vp, vp, ctypes.c_uint64]),
     ("lfb_kernel_launches", ctypes.c_uint64, []),
     ("lfb_tree_slot_tape", ctypes.c_int, [tree_t, u32p, i32p, u32p, fp, u32p, ctypes.POINTER(vp)]),
 ]

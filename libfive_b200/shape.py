@@ -188,10 +188,9 @@ def mesh_arrays(mesh_p, delete=True):
     """Copies a libfive_mesh* into numpy (verts float32 [N,3], tris uint32 [M,3])."""
     m = mesh_p[0]
     nv, nt = m.vert_count, m.tri_count
-    verts = np.ctypeslib.as_array(ctypes.cast(m.verts, ctypes.POINTER(ctypes.c_float)),
-                                  shape=(nv * 3,)).reshape(nv, 3).copy() if nv else np.zeros((0, 3), np.float32)
-    tris = np.ctypeslib.as_array(ctypes.cast(m.tris, ctypes.POINTER(ctypes.c_uint32)),
-                                 shape=(nt * 3,)).reshape(nt, 3).copy() if nt else np.zeros((0, 3), np.uint32)
+    verts, tris = np.empty((nv, 3), np.float32), np.empty((nt, 3), np.uint32)
+    for to, src in ((verts, m.verts), (tris, m.tris)):
+        _lib().lfb_host_copy(to.ctypes.data, src, to.nbytes)
     if delete:
         _lib().libfive_mesh_delete(mesh_p)
     return verts, tris
