@@ -3,10 +3,13 @@
 // mesher.
 //
 //  * Quadtree build (DCWorkerPool<2>::build, DCTree<2>::evalInterval,
-//    dc_tree.inl:94-128): level by level, one thread per cell evaluates the
-//    cell's interval over its parent's pruned register tape and prunes it
-//    for its children (Tape::push as liveness, like the mesher's group
-//    kernel), with the interval register file in global scratch.
+//    dc_tree.inl:94-128), level by level.  The first levels have few cells
+//    with long tapes and run the mesher's list kernels (interval_lists.cuh:
+//    a block or a warp works on a cell's independent clauses at once; z is
+//    an axis whose region is one point); deeper, one thread per cell
+//    evaluates the cell's interval over its parent's pruned register tape
+//    and prunes it for its children (Tape::push as liveness), with the
+//    interval register file in global scratch.
 //  * Leaves (DCTree<2>::evalLeaf, dc_tree.inl:131-552 with N = 2): one warp
 //    per cell; corners, edge search (four rounds of 16 samples per edge,
 //    lanes over samples), gradients and features at the brackets, the
@@ -18,6 +21,8 @@
 //    writes one segment per sign-changing minimal edge.
 //  * Contours::collect (contours.cpp:118-184): the segments are welded into
 //    polylines on the host, in the reference's order of operations.
+#include <cub/cub.cuh>
+
 #include <algorithm>
 #include <cmath>
 #include <list>
@@ -29,6 +34,7 @@
 #include "dc_device.cuh"
 #include "dc_features.cuh"
 #include "eval_kernels.cuh"
+#include "interval_lists.cuh"
 #include "libfive_b200.h"
 
 namespace lfb {
@@ -224,8 +230,15 @@ k_q_interval(QIntervalArgs A)
 
 /// Children of the branch cells of depth d: four each, in the order of
 /// Region::subdivide (bit 0 = x upper half, bit 1 = y upper half), with
-/// their parent's pruned tape.
-__global__ void k_q_children(QTree t, int d, const uint32_t* scan, const TapeRef* out_tape)
+/// their parent's pruned tape.  Levels in list form (lists not null) also
+/// get the coordinates, tapes and lists that the list kernels read.
+struct QListLevel {
+    uint64_t* coords;          // cells of depth d + 1
+    TapeRef* group_tape;       // one per four of them
+    ListRef* group_list;
+};
+__global__ void k_q_children(QTree t, int d, const uint32_t* scan, const TapeRef* out_tape,
+                             const ListRef* out_list, QListLevel next)
 {
     const QLevel& lv = t.lv[d];
     const QLevel& nx = t.lv[d + 1];
@@ -240,15 +253,21 @@ __global__ void k_q_children(QTree t, int d, const uint32_t* scan, const TapeRef
     lv.child[i] = c0;
     const uint2 p = lv.xy[i];
     for (uint32_t k = 0; k < 4; ++k) {
-        nx.xy[c0 + k] = make_uint2(2 * p.x + (k & 1), 2 * p.y + ((k >> 1) & 1));
+        const uint2 q = make_uint2(2 * p.x + (k & 1), 2 * p.y + ((k >> 1) & 1));
+        nx.xy[c0 + k] = q;
         nx.tape[c0 + k] = out_tape[i];
+        if (out_list) next.coords[c0 + k] = pack_coords(q.x, q.y, 0);
+    }
+    if (out_list) {
+        next.group_tape[scan[i]] = out_tape[i];
+        next.group_list[scan[i]] = out_list[i];
     }
 }
 
 __global__ void k_q_branch_flags(const uint8_t* type, uint32_t n, uint32_t* flags)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flags[i] = type[i] == CELL_BRANCH ? 1u : 0u;
+    if (i <= n) flags[i] = i < n && type[i] == CELL_BRANCH ? 1u : 0u;
 }
 
 ////////////////////////////////////////////////////////////////////////////////
@@ -852,6 +871,43 @@ bool upload_tables2()
 
 }  // namespace
 
+namespace {
+
+/// Device buffers of the contourer, kept between calls (allocating them took
+/// a third of a slice): one call at a time, on one device.
+struct ContourBuffers {
+    enum Key {
+        ARENA, CTR, RLO, RHI, RNAN, LIVE, DEC, OUT_TAPE, SCAN, FLAGS, REGS, FEATWS, FS, RECS,
+        TASKS_A, TASKS_B, SEGS, CREGS, SCANTMP, LISTS_A, LISTS_B, CELL_LIST, COORDS_A, COORDS_B,
+        GTAPE_A, GTAPE_B, GLIST_A, GLIST_B, WIDE, LEVEL
+    };
+    static constexpr size_t kKeepBytes = size_t(4) << 30;   // given back beyond
+    std::mutex mu;
+    int device = -1;
+    std::map<int, DevBuf> bufs;
+    template <class T>
+    T* get(int key, size_t count)
+    {
+        DevBuf& b = bufs[key];
+        b.ordered = true;   // from the device's memory pool, on the default stream
+        return b.reserve(std::max<size_t>(count, 1) * sizeof(T)) ? b.as<T>() : nullptr;
+    }
+    void trim()
+    {
+        size_t total = 0;
+        for (const auto& b : bufs) total += b.second.bytes;
+        if (total > kKeepBytes) bufs.clear();
+    }
+};
+
+ContourBuffers& contour_buffers()
+{
+    static auto* b = new ContourBuffers;   // never destroyed, like the mesher's contexts
+    return *b;
+}
+
+}  // namespace
+
 /// Contours::collect (contours.cpp:118-184): directed segments welded into
 /// polylines, first by extending a polyline whose tail is the segment's
 /// start, else one whose head is its end, else starting a new one; then
@@ -926,31 +982,60 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
     const uint32_t leaf_warps = static_cast<uint32_t>(sms) * 8;
     cudaStream_t s = 0;
 
+    ContourBuffers& B = contour_buffers();
+    std::lock_guard<std::mutex> lock(B.mu);
+    int dev = 0;
+    if (!cuda_ok(cudaGetDevice(&dev), "device")) return LFB_E_CUDA;
+    if (B.device != dev) {
+        if (B.device >= 0) {
+            cudaSetDevice(B.device);
+            B.bufs.clear();
+            cudaSetDevice(dev);
+        }
+        B.device = dev;
+    }
+    struct Trim {
+        ContourBuffers& b;
+        ~Trim() { b.trim(); }
+    } trim{B};
+    using CB = ContourBuffers;
+
+    // The list kernels take the first levels, while there are fewer cells
+    // than kListCells: a thread a cell walks a tape clause by clause, 0.5 us
+    // a clause whatever the number of cells, and only the deeper levels'
+    // tapes are short.  Tapes that the list kernels do not take (more than
+    // kMaxTapeRegs registers, dependency chains too long for a list) start
+    // with a thread a cell.
+    constexpr uint32_t kListCells = 8192;
+    const bool lists_ok = bt.n && bt.n_regs <= kMaxTapeRegs && g.ensure_wide();
+    if (!lists_ok) clear_error();
+
     uint64_t arena_cap = std::max<uint64_t>(static_cast<uint64_t>(bt.n) * 64, 1u << 20);
+    uint64_t list_cap = 4ull * bt.n + 1024;
     uint32_t rec_cap = 1u << 16, task_cap = 1u << 18, seg_cap = 1u << 16;
-    for (int attempt = 0; attempt < 4; ++attempt) {
-        DevBuf b_arena, b_ctr, b_rlo, b_rhi, b_rnan, b_live, b_dec, b_out_tape, b_scan, b_flags;
-        DevBuf b_regs, b_featws, b_fs, b_recs, b_tasks_a, b_tasks_b, b_segs, b_cregs;
-        std::vector<DevBuf> lv_bufs(static_cast<size_t>(L) + 1);
+    for (int attempt = 0; attempt < 6; ++attempt) {
         const size_t tr_bytes = static_cast<size_t>(nregs) * T;
-        if (!b_arena.reserve(arena_cap * sizeof(RegClause)) || !b_ctr.reserve(64) ||
-            !b_rlo.reserve(tr_bytes * 4) || !b_rhi.reserve(tr_bytes * 4) ||
-            !b_rnan.reserve(tr_bytes) || !b_live.reserve(tr_bytes) ||
-            !b_dec.reserve(static_cast<size_t>(dec_cap) * T) ||
-            !b_regs.reserve(static_cast<size_t>(leaf_warps) * nregs * 4 * 32 * sizeof(float)) ||
-            !b_featws.reserve(static_cast<size_t>(leaf_warps) * bt.n_regs * kRegBlock * sizeof(float) + 16) ||
-            !b_fs.reserve(static_cast<size_t>(leaf_warps) * sizeof(FeatureScratch)) ||
-            !b_recs.reserve(static_cast<size_t>(rec_cap) * sizeof(QLeaf)) ||
-            !b_tasks_a.reserve(static_cast<size_t>(task_cap) * sizeof(QTask)) ||
-            !b_tasks_b.reserve(static_cast<size_t>(task_cap) * sizeof(QTask)) ||
-            !b_segs.reserve(static_cast<size_t>(seg_cap) * sizeof(uint2)) ||
-            !b_cregs.reserve(tr_bytes * 4)) {
+        RegClause* arena = B.get<RegClause>(CB::ARENA, arena_cap);
+        unsigned long long* ctr = B.get<unsigned long long>(CB::CTR, 8);
+        float* rlo = B.get<float>(CB::RLO, tr_bytes);
+        float* rhi = B.get<float>(CB::RHI, tr_bytes);
+        uint8_t* rnan = B.get<uint8_t>(CB::RNAN, tr_bytes);
+        uint8_t* live = B.get<uint8_t>(CB::LIVE, tr_bytes);
+        uint8_t* dec = B.get<uint8_t>(CB::DEC, static_cast<size_t>(dec_cap) * T);
+        float* lregs = B.get<float>(CB::REGS, static_cast<size_t>(leaf_warps) * nregs * 4 * 32);
+        float* featws = B.get<float>(CB::FEATWS, static_cast<size_t>(leaf_warps) * bt.n_regs * kRegBlock + 4);
+        FeatureScratch* fs = B.get<FeatureScratch>(CB::FS, leaf_warps);
+        QLeaf* recs_d = B.get<QLeaf>(CB::RECS, rec_cap);
+        QTask* tasks_a = B.get<QTask>(CB::TASKS_A, task_cap);
+        QTask* tasks_b = B.get<QTask>(CB::TASKS_B, task_cap);
+        uint2* segs_d = B.get<uint2>(CB::SEGS, seg_cap);
+        float* cregs = B.get<float>(CB::CREGS, tr_bytes);
+        if (!arena || !ctr || !rlo || !rhi || !rnan || !live || !dec || !lregs || !featws || !fs ||
+            !recs_d || !tasks_a || !tasks_b || !segs_d || !cregs) {
             return LFB_E_CUDA;
         }
-        RegClause* arena = b_arena.as<RegClause>();
-        unsigned long long* ctr = b_ctr.as<unsigned long long>();
         // ctr[0] arena top, [1] record top (u32), [2] status (u32), [3] task
-        // count, [4] segment count
+        // count, [4] segment count, [5] list top, [6] work counter (u32)
         unsigned long long* arena_top = ctr;
         uint32_t* rec_top = reinterpret_cast<uint32_t*>(ctr + 1);
         uint32_t* status = reinterpret_cast<uint32_t*>(ctr + 2);
@@ -971,8 +1056,8 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         auto alloc_level = [&](int d, uint32_t n) {
             const size_t m = std::max<uint32_t>(n, 1);
             const size_t bytes = m * (sizeof(uint2) + sizeof(TapeRef) + 1 + 4 + 4) + 64;
-            if (!lv_bufs[d].reserve(bytes)) return false;
-            unsigned char* p = lv_bufs[d].as<unsigned char>();
+            unsigned char* p = B.get<unsigned char>(CB::LEVEL + d, bytes);
+            if (!p) return false;
             QLevel& q = t.lv[d];
             q.n = n;
             q.xy = reinterpret_cast<uint2*>(p);
@@ -988,7 +1073,55 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         cudaMemcpyAsync(t.lv[0].xy, &root_xy, sizeof(root_xy), cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(t.lv[0].tape, &root_ref, sizeof(root_ref), cudaMemcpyHostToDevice, s);
 
+        // List form: the octree that the kernels see (only the level at work
+        // is filled in), its scratch and the two list arenas.
+        bool lists = lists_ok;
+        WideArgs W{};
+        uint32_t wide_warps = 0;
+        QListLevel ql[2] = {};
+        if (lists) {
+            const uint64_t per = wide_scratch_bytes(bt.n, 1);
+            wide_warps = static_cast<uint32_t>(std::max<uint64_t>(
+                             8, std::min<uint64_t>(static_cast<uint64_t>(sms) * 16, (512ull << 20) / per))) /
+                         8 * 8;
+            size_t zeroed = 0;
+            const size_t bytes = wide_scratch_bytes(bt.n, wide_warps, &zeroed);
+            unsigned char* w = B.get<unsigned char>(CB::WIDE, bytes);
+            if (!w) return LFB_E_CUDA;
+            wide_scratch_carve(W, w, bt.n, wide_warps);
+            cudaMemsetAsync(W.st2, 0, zeroed, s);
+            W.o.lo[0] = lo[0]; W.o.lo[1] = lo[1];
+            W.o.hi[0] = hi[0]; W.o.hi[1] = hi[1];
+            W.o.lo[2] = W.o.hi[2] = t.perp;
+            W.o.levels = L;
+            W.bt = bt;
+            W.n = bt.n;
+            W.root_list = {0u, bt.n, g.wide_root, 0u};
+            W.arena = arena;
+            W.arena_top = arena_top;
+            W.arena_cap = arena_cap;
+            W.out_top = ctr + 5;
+            W.out_cap = list_cap;
+            W.status = status;
+            W.next_cell = reinterpret_cast<uint32_t*>(ctr + 6);
+            W.group_shift = 2;
+            ql[0].coords = B.get<uint64_t>(CB::COORDS_A, 4 * kListCells);
+            ql[1].coords = B.get<uint64_t>(CB::COORDS_B, 4 * kListCells);
+            ql[0].group_tape = B.get<TapeRef>(CB::GTAPE_A, kListCells);
+            ql[1].group_tape = B.get<TapeRef>(CB::GTAPE_B, kListCells);
+            ql[0].group_list = B.get<ListRef>(CB::GLIST_A, kListCells);
+            ql[1].group_list = B.get<ListRef>(CB::GLIST_B, kListCells);
+            if (!ql[0].coords || !ql[1].coords || !ql[0].group_tape || !ql[1].group_tape ||
+                !ql[0].group_list || !ql[1].group_list ||
+                !B.get<ListRef>(CB::CELL_LIST, kListCells) ||
+                !B.get<WideEntry>(CB::LISTS_A, list_cap) || !B.get<WideEntry>(CB::LISTS_B, list_cap)) {
+                return LFB_E_CUDA;
+            }
+            cudaMemsetAsync(ql[0].coords, 0, sizeof(uint64_t), s);
+        }
+
         // quadtree build, level by level
+        bool list_overflow = false, arena_overflow = false;
         for (int d = 0; d < L; ++d) {
             const uint32_t n = t.lv[d].n;
             if (n == 0) {
@@ -996,40 +1129,63 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
                 if (!alloc_level(d + 1, 0)) return LFB_E_CUDA;
                 continue;
             }
-            if (!b_out_tape.reserve(static_cast<size_t>(n) * sizeof(TapeRef)) ||
-                !b_flags.reserve(static_cast<size_t>(n + 1) * 4) ||
-                !b_scan.reserve(static_cast<size_t>(n + 1) * 4)) {
-                return LFB_E_CUDA;
+            TapeRef* out_tape = B.get<TapeRef>(CB::OUT_TAPE, n);
+            uint32_t* flags = B.get<uint32_t>(CB::FLAGS, n + 1);
+            uint32_t* scan = B.get<uint32_t>(CB::SCAN, n + 1);
+            size_t tmp_bytes = 0;
+            cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flags, scan, n + 1, s);
+            void* tmp = B.get<unsigned char>(CB::SCANTMP, tmp_bytes);
+            if (!out_tape || !flags || !scan || !tmp) return LFB_E_CUDA;
+            lists = lists && n < kListCells;
+            ListRef* cell_list = nullptr;
+            if (lists) {
+                LevelView& lv = W.o.lv[d];
+                cell_list = B.get<ListRef>(CB::CELL_LIST, n);
+                lv = LevelView{};
+                lv.n_cells = n;
+                lv.coords = ql[d & 1].coords;
+                lv.type = t.lv[d].type;
+                lv.cell_tape = out_tape;
+                lv.cell_list = cell_list;
+                lv.group_tape = ql[d & 1].group_tape;
+                lv.group_list = ql[d & 1].group_list;
+                W.in_lists = d == 0 ? g.d_wide
+                                    : B.get<WideEntry>(d & 1 ? CB::LISTS_B : CB::LISTS_A, list_cap);
+                W.out_lists = B.get<WideEntry>(d & 1 ? CB::LISTS_A : CB::LISTS_B, list_cap);
+                W.write_lists = d + 1 < L;
+                cudaMemsetAsync(ctr + 5, 0, 16, s);
+                if (!cuda_ok(launch_interval_lists(W, d, n, wide_warps, s), "contour intervals")) {
+                    return LFB_E_CUDA;
+                }
+            } else {
+                QIntervalArgs A{t, d, bt, arena, arena_top, arena_cap, out_tape, rlo, rhi,
+                                rnan, live, dec, dec_cap, T, status};
+                k_q_interval<<<std::min<uint32_t>(T / 256, (n + 255) / 256), 256, 0, s>>>(A);
             }
-            QIntervalArgs A{t, d, bt, arena, arena_top, arena_cap, b_out_tape.as<TapeRef>(),
-                            b_rlo.as<float>(), b_rhi.as<float>(), b_rnan.as<uint8_t>(),
-                            b_live.as<uint8_t>(), b_dec.as<uint8_t>(), dec_cap, T, status};
-            k_q_interval<<<T / 256, 256, 0, s>>>(A);
-            k_q_branch_flags<<<(n + 255) / 256, 256, 0, s>>>(t.lv[d].type, n, b_flags.as<uint32_t>());
+            k_q_branch_flags<<<(n + 256) / 256, 256, 0, s>>>(t.lv[d].type, n, flags);
             note_launches(2);
-            // exclusive scan of the branch flags on the host (quadtree
-            // levels are small; the counts decide the next level's size)
-            std::vector<uint32_t> flags(n);
-            if (!cuda_ok(cudaMemcpyAsync(flags.data(), b_flags.as<uint32_t>(), n * 4,
-                                         cudaMemcpyDeviceToHost, s), "download") ||
+            uint32_t n_branch = 0, st = 0;
+            if (!cuda_ok(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flags, scan, n + 1, s), "scan") ||
+                !cuda_ok(cudaMemcpyAsync(&n_branch, scan + n, 4, cudaMemcpyDeviceToHost, s), "download") ||
+                !cuda_ok(cudaMemcpyAsync(&st, status, 4, cudaMemcpyDeviceToHost, s), "download") ||
                 !cuda_ok(cudaStreamSynchronize(s), "contour intervals")) {
                 return LFB_E_CUDA;
             }
-            std::vector<uint32_t> scan(n + 1, 0);
-            for (uint32_t k = 0; k < n; ++k) scan[k + 1] = scan[k] + flags[k];
-            const uint32_t n_next = 4 * scan[n];
-            cudaMemcpyAsync(b_scan.as<uint32_t>(), scan.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s);
-            if (!alloc_level(d + 1, n_next)) return LFB_E_CUDA;
-            k_q_children<<<(n + 255) / 256, 256, 0, s>>>(t, d, b_scan.as<uint32_t>(),
-                                                         b_out_tape.as<TapeRef>());
+            list_overflow = (st & ST_LIST_OVERFLOW) != 0;
+            arena_overflow = (st & ST_ARENA_OVERFLOW) != 0;
+            if (list_overflow || arena_overflow) break;
+            if (!alloc_level(d + 1, 4 * n_branch)) return LFB_E_CUDA;
+            k_q_children<<<(n + 255) / 256, 256, 0, s>>>(t, d, scan, out_tape, cell_list, ql[(d + 1) & 1]);
             note_launches(1);
             if (!cuda_ok(cudaGetLastError(), "contour intervals")) return LFB_E_CUDA;
         }
+        if (list_overflow) list_cap *= 4;
+        if (arena_overflow) arena_cap *= 4;
+        if (list_overflow || arena_overflow) continue;
 
         // leaves at the finest depth
         if (t.lv[L].n) {
-            QLeafArgs A{t, bt, arena, b_regs.as<float>(), nregs, b_featws.as<float>(),
-                        b_fs.as<FeatureScratch>(), b_recs.as<QLeaf>(), rec_top, rec_cap, status};
+            QLeafArgs A{t, bt, arena, lregs, nregs, featws, fs, recs_d, rec_top, rec_cap, status};
             const uint32_t blocks = std::min<uint32_t>(leaf_warps / kLeafWarps,
                                                        (t.lv[L].n + kLeafWarps - 1) / kLeafWarps);
             k_q_leaf<<<std::max<uint32_t>(blocks, 1), 32 * kLeafWarps, 0, s>>>(A);
@@ -1037,8 +1193,8 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         }
         // collapse, bottom-up
         for (int d = L - 1; d >= 0; --d) {
-            QCollapseArgs C{t, d, bt, arena, b_recs.as<QLeaf>(), rec_top, rec_cap, max_err,
-                            b_cregs.as<float>(), T, status};
+            QCollapseArgs C{t, d, bt, arena, recs_d, rec_top, rec_cap, max_err,
+                            cregs, T, status};
             k_q_collapse<<<T / 256, 256, 0, s>>>(C);
             note_launches(1);
         }
@@ -1052,14 +1208,14 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         }
 
         // dual walk
-        QDualArgs D{t, b_recs.as<QLeaf>(), b_tasks_a.as<QTask>(), n_tasks, task_cap,
-                    b_segs.as<uint2>(), n_segs, seg_cap, status};
+        QDualArgs D{t, recs_d, tasks_a, n_tasks, task_cap,
+                    segs_d, n_segs, seg_cap, status};
         for (int d = 0; d < L; ++d) {
             if (t.lv[d].n) k_q_dual_init<<<(t.lv[d].n + 255) / 256, 256, 0, s>>>(D, d);
             note_launches(1);
         }
-        QTask* qa = b_tasks_a.as<QTask>();
-        QTask* qb = b_tasks_b.as<QTask>();
+        QTask* qa = tasks_a;
+        QTask* qb = tasks_b;
         uint32_t n_in = 0;
         cudaMemcpyAsync(&n_in, n_tasks, 4, cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(&st, status, 4, cudaMemcpyDeviceToHost, s);
@@ -1087,9 +1243,9 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         if (!cuda_ok(cudaStreamSynchronize(s), "contour walk")) return LFB_E_CUDA;
         std::vector<uint2> segs(ns);
         std::vector<QLeaf> recs(nr);
-        if ((ns && !cuda_ok(cudaMemcpy(segs.data(), b_segs.as<uint2>(), ns * sizeof(uint2),
+        if ((ns && !cuda_ok(cudaMemcpy(segs.data(), segs_d, ns * sizeof(uint2),
                                        cudaMemcpyDeviceToHost), "download")) ||
-            (nr && !cuda_ok(cudaMemcpy(recs.data(), b_recs.as<QLeaf>(), nr * sizeof(QLeaf),
+            (nr && !cuda_ok(cudaMemcpy(recs.data(), recs_d, nr * sizeof(QLeaf),
                                        cudaMemcpyDeviceToHost), "download"))) {
             return LFB_E_CUDA;
         }

@@ -33,6 +33,7 @@
 #include "dc_device.cuh"
 #include "dc_features.cuh"
 #include "eval_kernels.cuh"
+#include "interval_lists.cuh"
 #include "leaf_interp.cuh"
 
 namespace lfb {
@@ -50,7 +51,6 @@ __constant__ DcTables c_tab;
 // memory, that of longer lists in a per-warp global scratch slice.
 
 constexpr uint32_t kWideSmemSlots = 512;
-constexpr uint32_t kMaxTapeRegs = 400;
 constexpr uint32_t kRenumberMax = kWideSmemSlots;   // tapes up to this length get compact registers
 constexpr uint32_t kGroupModeCells = 8192;          // cells per level from which k_interval_group runs
 constexpr uint32_t kBlockModeCells = 2048;          // cells per level up to which k_interval_block runs
@@ -63,34 +63,6 @@ struct WideSmem {
     uint8_t SN[kWideSmemSlots + 3];    // slot maybe-NaN flags
     uint8_t pst[kWideSmemSlots];       // entry state for the children
     uint8_t live[kWideSmemSlots];      // entry still needed by the children
-};
-
-struct WideArgs {
-    Octree o;
-    DevTape bt;
-    uint32_t n;                    // clauses of the unpruned tape
-    const WideEntry* in_lists;     // lists of this depth's groups
-    ListRef root_list;             // the unpruned list (depth 0)
-    WideEntry* out_lists;          // lists handed to the next depth
-    unsigned long long* out_top;
-    uint64_t out_cap;
-    int write_lists;
-    RegClause* arena;              // register tapes
-    unsigned long long* arena_top;
-    uint64_t arena_cap;
-    // Per-warp global scratch: slot state of long lists, and the two-level
-    // bitmap of clause states that orders the register tape (zero between
-    // cells).
-    float2* S;                     // [warps][n + 3]
-    uint8_t* SN;                   // [warps][n + 3]
-    uint8_t* pst;                  // [warps][n]
-    uint8_t* live;                 // [warps][n]
-    uint32_t* newpos;              // [warps][n]
-    uint32_t* st2;                 // [warps][nw]   2-bit state per clause
-    uint32_t* l1;                  // [warps][nw1]  non-zero words of st2
-    uint32_t* wl;                  // [warps][nw]   word list
-    uint32_t* status;
-    uint32_t* next_cell;           // work counter (zero at launch)
 };
 
 __device__ __forceinline__ Iv wide_fetch(uint32_t kind, uint32_t idx,
@@ -300,8 +272,8 @@ k_interval_wide(WideArgs A, int d)
             P = A.root_list;
             T = root_tape_ref(bt);
         } else {
-            P = lv.group_list[i >> 3];
-            T = lv.group_tape[i >> 3];
+            P = lv.group_list[i >> A.group_shift];
+            T = lv.group_tape[i >> A.group_shift];
         }
         const uint4* PL = reinterpret_cast<const uint4*>(A.in_lists + P.off);
         const bool small = P.len <= kWideSmemSlots;
@@ -604,8 +576,8 @@ k_interval_block(WideArgs A, int d)
             P = A.root_list;
             T = root_tape_ref(bt);
         } else {
-            P = lv.group_list[i >> 3];
-            T = lv.group_tape[i >> 3];
+            P = lv.group_list[i >> A.group_shift];
+            T = lv.group_tape[i >> A.group_shift];
         }
         const uint4* PL = reinterpret_cast<const uint4*>(A.in_lists + P.off);
         if (tid < 3) {
@@ -2687,6 +2659,28 @@ bool debug_levels()
     return on;
 }
 
+}  // namespace
+
+cudaError_t launch_interval_lists(const WideArgs& W, int d, uint32_t n_cells, uint32_t scratch_warps,
+                                  cudaStream_t s)
+{
+    if (n_cells <= block_mode_cells()) {
+        const uint32_t blocks = std::min<uint32_t>(
+            std::min<uint32_t>(scratch_warps, device_sm_count() * 2), n_cells);
+        k_interval_block<<<std::max<uint32_t>(blocks, 1), kBlockThreads, 0, s>>>(W, d);
+    } else {
+        const size_t smem = sizeof(WideSmem) * 8;
+        if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_wide), smem)) {
+            return cudaErrorInvalidValue;
+        }
+        const uint32_t warps = std::min<uint32_t>(scratch_warps, (n_cells + 7) / 8 * 8);
+        k_interval_wide<<<warps / 8, 256, smem, s>>>(W, d);
+    }
+    return cudaGetLastError();
+}
+
+namespace {
+
 template <class T>
 bool exclusive_scan(Workspace& ws, const T* in, T* out, uint32_t n, cudaStream_t s)
 {
@@ -3064,10 +3058,6 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         cudaMemsetAsync(wSt2, 0, scratch_warps * nw16 * 4, s);
         cudaMemsetAsync(wL1, 0, scratch_warps * nw1 * 4, s);
     }
-    const size_t wide_smem = sizeof(WideSmem) * 8;
-    if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_wide), wide_smem)) {
-        return LFB_E_CUDA;
-    }
     // Two list arenas, one per parity of depth: depth d reads the lists of
     // its groups from one and writes its children's lists to the other.
     const int list_key[2] = {K_LIST_A, K_LIST_B};
@@ -3140,6 +3130,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             W.wl = wWl;
             W.status = status;
             W.next_cell = reinterpret_cast<uint32_t*>(counters + 6);
+            W.group_shift = 3;
             cudaMemsetAsync(W.next_cell, 0, sizeof(uint32_t), s);
             cudaMemsetAsync(list_top, 0, sizeof(unsigned long long), s);
             if (group_mode) {
@@ -3147,13 +3138,9 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
                             nregs_d, status, W.next_cell};
                 const uint32_t blocks = std::min<uint32_t>(group_warps / 4, (lv.n_groups + 3) / 4);
                 k_interval_group<<<std::max<uint32_t>(blocks, 1), 128, group_smem, s>>>(G, d);
-            } else if (lv.n_cells <= block_mode_cells()) {
-                const uint32_t blocks = std::min<uint32_t>(
-                    std::min<uint32_t>(scratch_warps, device_sm_count() * 2), lv.n_cells);
-                k_interval_block<<<std::max<uint32_t>(blocks, 1), kBlockThreads, 0, s>>>(W, d);
-            } else {
-                const uint32_t warps = std::min<uint32_t>(scratch_warps, (lv.n_cells + 7) / 8 * 8);
-                k_interval_wide<<<warps / 8, 256, wide_smem, s>>>(W, d);
+            } else if (!cuda_ok(launch_interval_lists(W, d, lv.n_cells, scratch_warps, s),
+                                "interval kernel")) {
+                return LFB_E_CUDA;
             }
             ++n_launch;
             if (!cuda_ok(cudaGetLastError(), "interval kernel")) return LFB_E_CUDA;
