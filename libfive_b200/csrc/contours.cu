@@ -151,7 +151,7 @@ k_q_interval(QIntervalArgs A)
             const uint32_t ro = raw.x >> 16;
             const Iv a = fetch(kinds & 3, raw.y & 0xffff);
             const Iv b = fetch((kinds >> 2) & 3, raw.y >> 16);
-            const Iv r = iv_apply(o, a, b);
+            const Iv r = iv_eval(o, a, b);
             if (o == op::MIN || o == op::MAX) {
                 uint8_t keep = 0;   // 0 both, 1 a, 2 b
                 if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;

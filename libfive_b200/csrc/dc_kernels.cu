@@ -26,6 +26,7 @@
 // reference's scalar code, so the octree and the mesh are reproducible.
 #include <cub/cub.cuh>
 #include <sys/mman.h>
+#include <type_traits>
 #include <thread>
 #include <cstdlib>
 #include <cstring>
@@ -65,22 +66,34 @@ struct WideSmem {
     uint8_t live[kWideSmemSlots];      // entry still needed by the children
 };
 
-__device__ __forceinline__ Iv wide_fetch(uint32_t kind, uint32_t idx,
-                                         const float2* S, const uint8_t* SN,
-                                         const float* __restrict__ cp)
+__device__ __forceinline__ Iv wide_fetch(uint32_t kind, uint32_t idx, float c, const float2* S,
+                                         const uint8_t* SN)
 {
     if (kind == OPND_REG) {
         const float2 v = S[idx];
         return {v.x, v.y, SN[idx] != 0};
     }
-    const float v = __ldg(cp + idx);
-    return iv_make(v, v);
+    return iv_make(c, c);
+}
+
+/// The values of a list entry's constant and free-variable operands, loaded
+/// with the entry so that they are at hand when its level comes.
+struct WideConsts {
+    float a, b;
+};
+__device__ __forceinline__ WideConsts wide_consts(const uint4& e, const float* __restrict__ cp)
+{
+    const uint32_t kinds = (e.x >> 8) & 0xf;
+    WideConsts c{0.0f, 0.0f};
+    if ((kinds & 3) != OPND_REG) c.a = __ldg(cp + e.y);
+    if ((kinds >> 2) != OPND_REG) c.b = __ldg(cp + e.z);
+    return c;
 }
 
 /// Interval of list entry k, stored in slot 3 + k, and the entry's state for
 /// the cell's children; returns whether a min/max got decided
 /// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167).
-__device__ __forceinline__ bool wide_forward(const uint4& e, uint32_t k, const float* cp,
+__device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c, uint32_t k,
                                              float2* S, uint8_t* SN, uint8_t* pst)
 {
     const uint8_t o = e.x & 0xff;
@@ -90,13 +103,13 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, uint32_t k, const f
     uint8_t ps = static_cast<uint8_t>(st);
     bool decided = false;
     if (st == WIDE_A) {
-        r = wide_fetch(kinds & 3, e.y, S, SN, cp);
+        r = wide_fetch(kinds & 3, e.y, c.a, S, SN);
     } else if (st == WIDE_B) {
-        r = wide_fetch((kinds >> 2) & 3, e.z, S, SN, cp);
+        r = wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN);
     } else {
-        const Iv a = wide_fetch(kinds & 3, e.y, S, SN, cp);
-        const Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, S, SN, cp) : a;
-        r = iv_apply(o, a, b);
+        const Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
+        const Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
+        r = iv_eval(o, a, b);
         if (o == op::MIN || o == op::MAX) {
             uint8_t keep = 0;   // 0 both, 1 a, 2 b
             if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;
@@ -300,12 +313,13 @@ k_interval_wide(WideArgs A, int d)
             const uint32_t k = ch * 32 + lane;
             const bool valid = k < P.len;
             const uint4 e = valid ? PL[k] : make_uint4(0, 0, 0, 0);
+            const WideConsts c = wide_consts(e, bt.cpool);
             const uint32_t lev = valid ? (e.x >> kWideLevelShift) : 0xffffffffu;
             const int last = static_cast<int>(min(31u, P.len - 1 - ch * 32));
             uint32_t l = __shfl_sync(full, lev, 0);
             const uint32_t lmax = __shfl_sync(full, lev, last);
             while (true) {
-                if (lev == l) changed |= wide_forward(e, k, bt.cpool, S, SN, pst);
+                if (lev == l) changed |= wide_forward(e, c, k, S, SN, pst);
                 __syncwarp();
                 if (l == lmax) break;
                 const uint32_t m = __ballot_sync(full, valid && lev > l);
@@ -313,7 +327,8 @@ k_interval_wide(WideArgs A, int d)
             }
         }
         changed = __any_sync(full, changed);
-        const Iv root = wide_fetch(bt.root_kind, P.root, S, SN, bt.cpool);
+        const float root_c = bt.root_kind == OPND_REG ? 0.0f : __ldg(bt.cpool + P.root);
+        const Iv root = wide_fetch(bt.root_kind, P.root, root_c, S, SN);
         const uint8_t state = iv_state(root);
         if (lane == 0) {
             lv.type[i] = state == ST_EMPTY ? CELL_EMPTY
@@ -520,33 +535,32 @@ k_interval_wide(WideArgs A, int d)
 // one cell: a wave of kBlockThreads consecutive entries at a time, stepping
 // through the levels the wave spans with a block barrier per level.  Same
 // results as k_interval_wide (lists, register tapes); tapes are not
-// renumbered (they are long at these depths).
+// renumbered (one thread renumbering 100 clauses took 40 us, longer than the
+// rest of a cell).
 
 constexpr int kBlockThreads = 512;
 constexpr int kBlockWarps = kBlockThreads / 32;
 
-/// Exclusive prefix over the block of one count per thread, and the total.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_tot,
-                                                    uint32_t& total)
+/// Exclusive prefix over the block's warps of one count per warp, and the
+/// total.
+__device__ __forceinline__ uint32_t warp_counts_scan(uint32_t count, uint32_t* warp_tot,
+                                                     uint32_t& total)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    if (lane == 0) warp_tot[warp] = count;
+    __syncthreads();
+    const uint32_t v = lane < kBlockWarps ? warp_tot[lane] : 0;
     const uint32_t incl = warp_incl_scan(v, lane);
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    uint32_t before = 0;
-    total = 0;
-    for (int w = 0; w < kBlockWarps; ++w) {
-        const uint32_t t = warp_tot[w];
-        if (w < warp) before += t;
-        total += t;
-    }
-    __syncthreads();
-    return before + incl - v;
+    total = __shfl_sync(0xffffffffu, incl, 31);
+    return __shfl_sync(0xffffffffu, incl - v, warp);
 }
 
-__global__ void __launch_bounds__(kBlockThreads)
-k_interval_block(WideArgs A, int d)
+__global__ void __launch_bounds__(kBlockThreads, 2)
+k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
 {
+    extern __shared__ __align__(16) unsigned char bsm[];
+    __shared__ uint32_t lev_of[2][2];   // levels of a wave's first and last entry
     __shared__ uint32_t warp_tot[kBlockWarps];
     __shared__ unsigned long long bcast;
     __shared__ uint32_t cell;
@@ -555,14 +569,7 @@ k_interval_block(WideArgs A, int d)
     const LevelView& lv = o.lv[d];
     const DevTape& bt = A.bt;
     const uint32_t n = A.n;
-    const uint32_t nw = (n + 15) / 16;
     const size_t slot = blockIdx.x;
-    float2* S = A.S + slot * (n + 3);
-    uint8_t* SN = A.SN + slot * (n + 3);
-    uint8_t* pst = A.pst + slot * n;
-    uint8_t* live = A.live + slot * n;
-    uint32_t* newpos = A.newpos + slot * n;
-    uint32_t* st2 = A.st2 + slot * nw;
 
     while (true) {
         if (tid == 0) cell = atomicAdd(A.next_cell, 1u);
@@ -580,6 +587,39 @@ k_interval_block(WideArgs A, int d)
             T = lv.group_tape[i >> A.group_shift];
         }
         const uint4* PL = reinterpret_cast<const uint4*>(A.in_lists + P.off);
+        auto work = [&](auto in_smem) {
+        constexpr bool SM = decltype(in_smem)::value;
+        float2* S;
+        uint8_t *SN, *pst, *live, *cstate;
+        uint32_t* newpos;
+        if constexpr (SM) {
+            S = reinterpret_cast<float2*>(bsm);
+            newpos = reinterpret_cast<uint32_t*>(bsm);   // once S has served
+            cstate = bsm + 4 * smem_slots;
+            SN = bsm + 8 * (smem_slots + 3);
+            pst = SN + smem_slots + 3;
+            live = pst + smem_slots;
+        } else {
+            S = A.S + slot * (n + 3);
+            SN = A.SN + slot * (n + 3);
+            pst = A.pst + slot * n;
+            live = A.live + slot * n;
+            newpos = A.newpos + slot * n;
+            cstate = reinterpret_cast<uint8_t*>(S);
+        }
+        // The wave's entry of this thread, fetched while the wave before it
+        // is at work, with its constants and (by the wave's first and last
+        // entries) the levels that the wave spans.
+        const uint32_t nwaves = (P.len + kBlockThreads - 1) / kBlockThreads;
+        auto fetch = [&](uint32_t w, uint4& e) {
+            const uint32_t k = w * kBlockThreads + tid;
+            if (w >= nwaves || k >= P.len) return;
+            e = __ldg(PL + k);
+            if (tid == 0) lev_of[w & 1][0] = e.x >> kWideLevelShift;
+            if (k + 1 == P.len || tid == kBlockThreads - 1) lev_of[w & 1][1] = e.x >> kWideLevelShift;
+        };
+        uint4 e{}, e_next{};
+        fetch(0, e);
         if (tid < 3) {
             double blo[3], bhi[3];
             cell_bounds(o, d, lv.coords[i], blo, bhi);
@@ -591,29 +631,31 @@ k_interval_block(WideArgs A, int d)
         __syncthreads();
 
         // Forward pass: waves of consecutive entries, levels in order.
-        const uint32_t nwaves = (P.len + kBlockThreads - 1) / kBlockThreads;
         bool changed = false;
+        WideConsts c = wide_consts(e, bt.cpool), c_next{};
         for (uint32_t w = 0; w < nwaves; ++w) {
-            const uint32_t b0 = w * kBlockThreads;
-            const uint32_t k = b0 + tid;
-            const bool valid = k < P.len;
-            const uint4 e = valid ? PL[k] : make_uint4(0, 0, 0, 0);
-            const uint32_t lev = valid ? (e.x >> kWideLevelShift) : 0xffffffffu;
-            const uint32_t lf = PL[b0].x >> kWideLevelShift;
-            const uint32_t ll = PL[min(b0 + kBlockThreads, P.len) - 1].x >> kWideLevelShift;
+            const uint32_t k = w * kBlockThreads + tid;
+            const uint32_t lf = lev_of[w & 1][0], ll = lev_of[w & 1][1];
+            const uint32_t lev = k < P.len ? (e.x >> kWideLevelShift) : 0xffffffffu;
+            e_next = make_uint4(0, 0, 0, 0);
+            fetch(w + 1, e_next);
+            c_next = wide_consts(e_next, bt.cpool);
             for (uint32_t l = lf; l <= ll; ++l) {
-                if (lev == l) changed |= wide_forward(e, k, bt.cpool, S, SN, pst);
+                if (lev == l) changed |= wide_forward(e, c, k, S, SN, pst);
                 __syncthreads();
             }
+            e = e_next;
+            c = c_next;
         }
         changed = __syncthreads_or(changed) != 0;
-        const Iv root = wide_fetch(bt.root_kind, P.root, S, SN, bt.cpool);
+        const float root_c = bt.root_kind == OPND_REG ? 0.0f : __ldg(bt.cpool + P.root);
+        const Iv root = wide_fetch(bt.root_kind, P.root, root_c, S, SN);
         const uint8_t state = iv_state(root);
         if (tid == 0) {
             lv.type[i] = state == ST_EMPTY ? CELL_EMPTY
                        : state == ST_FILLED ? CELL_FILLED : CELL_BRANCH;
         }
-        if (state != ST_AMBIGUOUS) continue;
+        if (state != ST_AMBIGUOUS) return;
 
         if (root.nan || !changed) {
             // The children keep this tape; its list moves to the next arena.
@@ -635,57 +677,68 @@ k_interval_block(WideArgs A, int d)
                 lv.cell_list[i] = {off, P.len, P.root, 0u};
                 lv.cell_tape[i] = T;
             }
-            continue;
+            return;
         }
 
         // Backward liveness pass: waves in reverse, levels decreasing.
         if (tid == 0 && bt.root_kind == OPND_REG && P.root >= 3) live[P.root - 3] = 1;
+        fetch(nwaves - 1, e);
         __syncthreads();
-        for (int w = static_cast<int>(nwaves) - 1; w >= 0; --w) {
-            const uint32_t b0 = w * kBlockThreads;
-            const uint32_t k = b0 + tid;
+        for (uint32_t w = nwaves; w-- > 0;) {
+            const uint32_t k = w * kBlockThreads + tid;
+            const uint32_t lf = lev_of[w & 1][0], ll = lev_of[w & 1][1];
             const bool valid = k < P.len;
-            const uint4 e = valid ? PL[k] : make_uint4(0, 0, 0, 0);
             const uint32_t lev = valid ? (e.x >> kWideLevelShift) : 0xffffffffu;
-            const uint32_t lf = PL[b0].x >> kWideLevelShift;
-            const uint32_t ll = PL[min(b0 + kBlockThreads, P.len) - 1].x >> kWideLevelShift;
+            fetch(w - 1, e_next);   // wave -1 is past the last: nothing
             for (uint32_t l = ll + 1; l-- > lf;) {
                 if (lev == l && live[k]) wide_mark(e, pst[k], live);
                 __syncthreads();
             }
+            e = e_next;
         }
 
-        // Child positions of the live entries and their 2-bit states.
-        uint32_t cnt = 0;
-        for (uint32_t w = 0; w < nwaves; ++w) {
-            const uint32_t k = w * kBlockThreads + tid;
-            const bool lv_ = k < P.len && live[k];
-            uint32_t tot = 0;
-            const uint32_t before = block_excl_scan(lv_ ? 1u : 0u, warp_tot, tot);
-            if (lv_) {
-                newpos[k] = cnt + before;
-                const uint32_t c = PL[k].w;
-                atomicOr(st2 + (c >> 4), static_cast<uint32_t>(pst[k]) << (2 * (c & 15)));
-            }
-            cnt += tot;
+        // Child positions of the live entries and, by clause, their states
+        // (for the register tape, which is in clause order).  Each warp takes
+        // a contiguous share of the entries: one block scan for all.
+        for (uint32_t k = tid; k < (n + 3) / 4; k += kBlockThreads) {
+            reinterpret_cast<uint32_t*>(cstate)[k] = 0;
         }
+        const unsigned full = 0xffffffffu;
+        const int lane = tid & 31, warp = tid >> 5;
+        const uint32_t lt_mask = (1u << lane) - 1;
+        const uint32_t share = (P.len + 32 * kBlockWarps - 1) / (32 * kBlockWarps) * 32;
+        const uint32_t k_end = min(P.len, share * (warp + 1));
+        uint32_t here = 0, cnt = 0;
+        for (uint32_t k0 = share * warp; k0 < k_end; k0 += 32) {
+            here += __popc(__ballot_sync(full, k0 + lane < k_end && live[k0 + lane]));
+        }
+        uint32_t at = warp_counts_scan(here, warp_tot, cnt);
+        for (uint32_t k0 = share * warp; k0 < k_end; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            const bool lv_ = k < k_end && live[k];
+            const uint32_t m = __ballot_sync(full, lv_);
+            if (lv_) {
+                newpos[k] = at + __popc(m & lt_mask);
+                cstate[__ldg(&PL[k].w)] = pst[k];
+            }
+            at += __popc(m);
+        }
+        if (tid == 0 && A.write_lists) bcast = atomicAdd(A.out_top, static_cast<unsigned long long>(cnt));
         __syncthreads();
         const uint32_t new_root = (bt.root_kind == OPND_REG && P.root >= 3)
                                       ? newpos[P.root - 3] + 3 : P.root;
         uint32_t loff = 0;
         if (A.write_lists) {
-            if (tid == 0) bcast = atomicAdd(A.out_top, static_cast<unsigned long long>(cnt));
-            __syncthreads();
             const unsigned long long o64 = bcast;
-            __syncthreads();
             const bool ok = o64 + cnt <= A.out_cap;
             if (!ok && tid == 0) atomicOr(A.status, ST_LIST_OVERFLOW);
             if (ok) {
                 loff = static_cast<uint32_t>(o64);
                 uint4* out = reinterpret_cast<uint4*>(A.out_lists + loff);
+#pragma unroll 2
                 for (uint32_t k = tid; k < P.len; k += kBlockThreads) {
+                    uint4 e = __ldg(PL + k);
                     if (!live[k]) continue;
-                    uint4 e = PL[k];
                     const uint32_t ps = pst[k];
                     const uint32_t kinds = (e.x >> 8) & 0xf;
                     const bool binary = dev_is_binary(e.x & 0xff);
@@ -701,63 +754,55 @@ k_interval_block(WideArgs A, int d)
             }
         }
 
-        // Register tape: live clauses in clause order (dense over the state
-        // words, which hold the whole tape at these depths).
-        uint32_t emit = 0;
-        for (uint32_t w = tid; w < nw; w += kBlockThreads) emit += wide_word_emits(st2[w], w, bt.clauses);
-        uint32_t etot = 0;
-        block_excl_scan(emit, warp_tot, etot);
+        // Register tape: live clauses in clause order, a contiguous share of
+        // the unpruned tape's clauses a warp.  A decided min / max is a copy,
+        // dropped when it is onto the same register.
+        const uint32_t cshare = (n + 32 * kBlockWarps - 1) / (32 * kBlockWarps) * 32;
+        const uint32_t c_end = min(n, cshare * (warp + 1));
+        auto clause_of = [&](uint32_t c, uint2& raw) -> bool {
+            const uint32_t ps = c < c_end ? cstate[c] : 0;
+            if (ps == 0) return false;
+            raw = __ldg(reinterpret_cast<const uint2*>(bt.clauses + c));
+            if (ps == WIDE_BOTH) return true;
+            const uint32_t kinds = (raw.x >> 8) & 0xff;
+            const uint32_t kk = ps == WIDE_A ? (kinds & 3) : ((kinds >> 2) & 3);
+            const uint32_t src = ps == WIDE_A ? (raw.y & 0xffff) : (raw.y >> 16);
+            const uint32_t ro = raw.x >> 16;
+            raw = make_uint2(OP_COPY | (kk << 8) | (ro << 16), src);
+            return !(kk == OPND_REG && src == ro);
+        };
+        uint32_t emit = 0, etot = 0;
+#pragma unroll 4
+        for (uint32_t c0 = cshare * warp; c0 < c_end; c0 += 32) {
+            uint2 raw;
+            emit += __popc(__ballot_sync(full, clause_of(c0 + lane, raw)));
+        }
+        uint32_t pos = warp_counts_scan(emit, warp_tot, etot);
         if (tid == 0) bcast = atomicAdd(A.arena_top, static_cast<unsigned long long>(etot));
         __syncthreads();
         const unsigned long long a64 = bcast;
-        __syncthreads();
         const bool aok = a64 + etot <= A.arena_cap;
         if (!aok && tid == 0) atomicOr(A.status, ST_ARENA_OVERFLOW);
-        uint32_t pos = static_cast<uint32_t>(a64);
-        const uint32_t nwwaves = (nw + kBlockThreads - 1) / kBlockThreads;
-        for (uint32_t ww = 0; ww < nwwaves; ++ww) {
-            const uint32_t w = ww * kBlockThreads + tid;
-            uint32_t word = 0, e_ = 0;
-            if (w < nw) {
-                word = st2[w];
-                e_ = wide_word_emits(word, w, bt.clauses);
-                st2[w] = 0;
-            }
-            uint32_t tot = 0;
-            uint32_t at = pos + block_excl_scan(e_, warp_tot, tot);
-            if (aok) {
-                while (word) {
-                    const int j = (__ffs(word) - 1) >> 1;
-                    const uint32_t ps = (word >> (2 * j)) & 3;
-                    word &= ~(3u << (2 * j));
-                    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(bt.clauses + w * 16 + j));
-                    if (ps == WIDE_BOTH) {
-                        *reinterpret_cast<uint2*>(A.arena + at++) = raw;
-                        continue;
-                    }
-                    const uint32_t kinds = (raw.x >> 8) & 0xff;
-                    const uint32_t kk = ps == WIDE_A ? (kinds & 3) : ((kinds >> 2) & 3);
-                    const uint32_t src = ps == WIDE_A ? (raw.y & 0xffff) : (raw.y >> 16);
-                    const uint32_t ro = raw.x >> 16;
-                    if (kk == OPND_REG && src == ro) continue;
-                    RegClause cc;
-                    cc.op = OP_COPY;
-                    cc.kinds = static_cast<uint8_t>(kk);
-                    cc.out = static_cast<uint16_t>(ro);
-                    cc.a = static_cast<uint16_t>(src);
-                    cc.b = 0;
-                    A.arena[at++] = cc;
-                }
-            }
-            pos += tot;
+        uint2* to = reinterpret_cast<uint2*>(A.arena + a64);
+        for (uint32_t c0 = cshare * warp; aok && c0 < c_end; c0 += 32) {
+            uint2 raw;
+            const bool emits = clause_of(c0 + lane, raw);
+            const uint32_t m = __ballot_sync(full, emits);
+            if (emits) to[pos + __popc(m & lt_mask)] = raw;
+            pos += __popc(m);
+        }
+        TapeRef out_t = T;
+        if (aok) {
+            out_t = {static_cast<uint32_t>(a64), etot, bt.n_regs,
+                     static_cast<uint32_t>(bt.root) | (static_cast<uint32_t>(bt.root_kind) << 16)};
         }
         if (tid == 0) {
             lv.cell_list[i] = {loff, cnt, new_root, 0u};
-            lv.cell_tape[i] = aok ? TapeRef{static_cast<uint32_t>(a64), etot, bt.n_regs,
-                                             static_cast<uint32_t>(bt.root) |
-                                                 (static_cast<uint32_t>(bt.root_kind) << 16)}
-                                  : T;
+            lv.cell_tape[i] = out_t;
         }
+        };
+        if (P.len <= smem_slots && n <= 4 * smem_slots) work(std::true_type{});
+        else work(std::false_type{});
         __syncthreads();
     }
 }
@@ -850,7 +895,7 @@ k_interval_group(GroupArgs A, int d)
             const uint32_t ro = raw.x >> 16;
             const Iv a = fetch(kinds & 3, raw.y & 0xffff);
             const Iv b = fetch((kinds >> 2) & 3, raw.y >> 16);
-            const Iv r = iv_apply(o_, a, b);
+            const Iv r = iv_eval(o_, a, b);
             if (o_ == op::MIN || o_ == op::MAX) {
                 uint8_t keep = 0;   // 0 both, 1 a, 2 b
                 if (a.lo > b.hi) keep = (o_ == op::MAX) ? 1 : 2;
@@ -2665,9 +2710,19 @@ cudaError_t launch_interval_lists(const WideArgs& W, int d, uint32_t n_cells, ui
                                   cudaStream_t s)
 {
     if (n_cells <= block_mode_cells()) {
-        const uint32_t blocks = std::min<uint32_t>(
-            std::min<uint32_t>(scratch_warps, device_sm_count() * 2), n_cells);
-        k_interval_block<<<std::max<uint32_t>(blocks, 1), kBlockThreads, 0, s>>>(W, d);
+        // Shared memory for the longest list a cell of this level can have
+        // up to a whole SM's, half of it where there are more cells than SMs
+        // (their lists are pruned): two blocks then share an SM.
+        const uint32_t sms = static_cast<uint32_t>(device_sm_count());
+        const uint32_t per_sm = n_cells <= sms ? 1 : 2;
+        const uint32_t slots = std::min<uint32_t>((W.n + 3) / 4 * 4, (216u * 1024 / per_sm - 2048) / 11 / 4 * 4);
+        const size_t smem = (11 * static_cast<size_t>(slots) + 27 + 15) / 16 * 16;
+        if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_block), smem)) {
+            return cudaErrorInvalidValue;
+        }
+        const uint32_t blocks = std::min<uint32_t>(std::min<uint32_t>(scratch_warps, sms * per_sm),
+                                                   n_cells);
+        k_interval_block<<<std::max<uint32_t>(blocks, 1), kBlockThreads, smem, s>>>(W, d, slots);
     } else {
         const size_t smem = sizeof(WideSmem) * 8;
         if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_wide), smem)) {

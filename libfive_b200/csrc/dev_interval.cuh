@@ -111,6 +111,26 @@ __device__ inline Iv iv_cos_bounds(float lo, float hi, int depth = 0)
     return {-1.0f, 1.0f, false};
 }
 
+__device__ __forceinline__ Iv iv_div(const Iv& a, const Iv& b)
+{
+    const bool u = a.nan || b.nan ||
+        ((a.lo == -LF_INF || a.hi == LF_INF) &&
+         (b.lo == -LF_INF || b.hi == LF_INF)) ||
+        (a.lo <= 0.0f && a.hi >= 0.0f && b.lo <= 0.0f && b.hi >= 0.0f);
+    if (b.lo <= 0.0f && b.hi >= 0.0f) return {-LF_INF, LF_INF, u};
+    if (iv_bad(a) || iv_bad(b)) return {LF_QNAN, LF_QNAN, u};
+    const float xl = a.lo, xu = a.hi, yl = b.lo, yu = b.hi;
+    if (xu < 0) {
+        if (yu < 0) return {__fdiv_rd(xu, yl), __fdiv_ru(xl, yu), u};
+        return {__fdiv_rd(xl, yl), __fdiv_ru(xu, yu), u};
+    } else if (xl < 0) {
+        if (yu < 0) return {__fdiv_rd(xu, yu), __fdiv_ru(xl, yu), u};
+        return {__fdiv_rd(xl, yl), __fdiv_ru(xu, yl), u};
+    }
+    if (yu < 0) return {__fdiv_rd(xu, yu), __fdiv_ru(xl, yl), u};
+    return {__fdiv_rd(xl, yu), __fdiv_ru(xu, yl), u};
+}
+
 __device__ __forceinline__ Iv iv_binary(uint8_t o, const Iv& a, const Iv& b)
 {
     const bool bad = iv_bad(a) || iv_bad(b);
@@ -163,24 +183,7 @@ __device__ __forceinline__ Iv iv_binary(uint8_t o, const Iv& a, const Iv& b)
             }
             return {0.0f, 0.0f, u};
         }
-        case op::DIV: {
-            const bool u = a.nan || b.nan ||
-                ((a.lo == -LF_INF || a.hi == LF_INF) &&
-                 (b.lo == -LF_INF || b.hi == LF_INF)) ||
-                (a.lo <= 0.0f && a.hi >= 0.0f && b.lo <= 0.0f && b.hi >= 0.0f);
-            if (b.lo <= 0.0f && b.hi >= 0.0f) return {-LF_INF, LF_INF, u};
-            if (bad) return {LF_QNAN, LF_QNAN, u};
-            const float xl = a.lo, xu = a.hi, yl = b.lo, yu = b.hi;
-            if (xu < 0) {
-                if (yu < 0) return {__fdiv_rd(xu, yl), __fdiv_ru(xl, yu), u};
-                return {__fdiv_rd(xl, yl), __fdiv_ru(xu, yu), u};
-            } else if (xl < 0) {
-                if (yu < 0) return {__fdiv_rd(xu, yu), __fdiv_ru(xl, yu), u};
-                return {__fdiv_rd(xl, yl), __fdiv_ru(xu, yl), u};
-            }
-            if (yu < 0) return {__fdiv_rd(xu, yu), __fdiv_ru(xl, yl), u};
-            return {__fdiv_rd(xl, yu), __fdiv_ru(xu, yl), u};
-        }
+        case op::DIV: return iv_div(a, b);
         case op::MIN:
         case op::MAX: {
             Iv r;
@@ -314,7 +317,7 @@ __device__ __forceinline__ Iv iv_binary(uint8_t o, const Iv& a, const Iv& b)
                     if (!(blo >= 0)) {
                         const float t = -bhi; bhi = -blo; blo = t;
                     }
-                    const Iv q = iv_binary(op::DIV, Iv{ulo, uhi, false}, Iv{blo, bhi, false});
+                    const Iv q = iv_div(Iv{ulo, uhi, false}, Iv{blo, bhi, false});
                     const int qi = static_cast<int>(floorf(q.lo));
                     if (qi == static_cast<int>(floorf(q.hi))) {
                         const Iv bq = iv_smul(static_cast<float>(qi), b.lo, b.hi);
@@ -458,6 +461,33 @@ __device__ __forceinline__ bool dev_is_binary(uint8_t o)
 __device__ __forceinline__ Iv iv_apply(uint8_t o, const Iv& a, const Iv& b)
 {
     return dev_is_binary(o) ? iv_binary(o, a, b) : iv_unary(o, a);
+}
+
+/// The operations with long bodies, out of line and by value (operands and
+/// result stay in registers).
+static __device__ __noinline__ Iv iv_rare(uint8_t o, Iv a, Iv b)
+{
+    return iv_apply(o, a, b);
+}
+
+/// iv_apply for the tape interpreters: the frequent operations inline, each
+/// its own case, the others in a call.  (With all of them inline the
+/// dispatch was a call through local memory per clause.)
+__device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
+{
+    switch (o) {
+        case op::ADD: return iv_binary(op::ADD, a, b);
+        case op::SUB: return iv_binary(op::SUB, a, b);
+        case op::MUL: return iv_binary(op::MUL, a, b);
+        case op::MIN: return iv_binary(op::MIN, a, b);
+        case op::MAX: return iv_binary(op::MAX, a, b);
+        case op::SQUARE: return iv_unary(op::SQUARE, a);
+        case op::SQRT: return iv_unary(op::SQRT, a);
+        case op::NEG: return iv_unary(op::NEG, a);
+        case op::ABS: return iv_unary(op::ABS, a);
+        case OP_COPY: return a;
+        default: return iv_rare(o, a, b);
+    }
 }
 
 /// Interval::state(): AMBIGUOUS when the value may be NaN.

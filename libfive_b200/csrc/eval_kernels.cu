@@ -174,7 +174,7 @@ k_intervals(DevTape t, uint32_t n,
                                          uint16_t ra, uint16_t rb) {
             const Iv a = fetch_i(kinds & 3, ra, R, N, tid, B, cp);
             const Iv bb = fetch_i((kinds >> 2) & 3, rb, R, N, tid, B, cp);
-            const Iv r = iv_apply(o, a, bb);
+            const Iv r = iv_eval(o, a, bb);
             R[ro * 2 * B + tid] = r.lo;
             R[ro * 2 * B + B + tid] = r.hi;
             N[ro * B + tid] = r.nan;

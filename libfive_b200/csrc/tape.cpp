@@ -217,14 +217,21 @@ bool build_wide_list(const RegTape& t, std::vector<WideEntry>& out,
         tmp[c] = e;
         slot_of[rc.out] = static_cast<uint32_t>(3 + c);
     }
-    // Counting sort by level, stable in clause order; then operands and the
-    // root are renamed from clause slots to list slots.
+    // Counting sort by level, each level by opcode (neighbouring lanes of a
+    // kernel then run the same operation) and stable in clause order; then
+    // operands and the root are renamed from clause slots to list slots.
     std::vector<uint32_t> start(max_level + 2, 0);
     for (size_t c = 0; c < n; ++c) ++start[level[3 + c] + 1];
     for (uint32_t l = 1; l < start.size(); ++l) start[l] += start[l - 1];
-    std::vector<uint32_t> pos(n);
+    std::vector<uint32_t> order(n), pos(n);
+    {
+        uint32_t by_op[256 + 1] = {0};
+        for (size_t c = 0; c < n; ++c) ++by_op[t.clauses[c].op + 1];
+        for (uint32_t o = 1; o <= 256; ++o) by_op[o] += by_op[o - 1];
+        for (size_t c = 0; c < n; ++c) order[by_op[t.clauses[c].op]++] = static_cast<uint32_t>(c);
+    }
     out.assign(n, WideEntry{});
-    for (size_t c = 0; c < n; ++c) {
+    for (uint32_t c : order) {
         pos[c] = start[level[3 + c]]++;
         out[pos[c]] = tmp[c];
     }

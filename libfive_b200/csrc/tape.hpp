@@ -98,7 +98,7 @@ enum : uint32_t { WIDE_BOTH = 1, WIDE_A = 2, WIDE_B = 3 };
 constexpr uint32_t kWideLevelShift = 14;
 constexpr uint32_t kWideMaxLevel = (1u << (32 - kWideLevelShift)) - 1;
 
-/// The register tape's clauses sorted by level (stable within a level), all
+/// The register tape's clauses sorted by level (by opcode within a level), all
 /// in state WIDE_BOTH, plus the list slot (or pool index) of the root.  Fails for
 /// tapes whose dependency chain is longer than kWideMaxLevel.
 bool build_wide_list(const RegTape& t, std::vector<WideEntry>& out,
