@@ -28,6 +28,7 @@
 #include <sys/mman.h>
 #include <type_traits>
 #include <thread>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 
@@ -2349,12 +2350,8 @@ __device__ void emit_edge(const DualArgs& A, int ax, const uint32_t ts[4])
     }
 }
 
-__global__ void __launch_bounds__(128)
-k_dual_round(DualArgs A, const DualTask* in, uint32_t n_in)
+__device__ __forceinline__ void dual_task(const DualArgs& A, const DualTask& task)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_in) return;
-    const DualTask task = in[t];
     const Octree& o = A.o;
     const int ax = task.axis;
     if (task.kind == TASK_CELL) {
@@ -2421,6 +2418,20 @@ k_dual_round(DualArgs A, const DualTask* in, uint32_t n_in)
     }
 }
 
+/// One round: the tasks that the round before it left (n_in; null: the root
+/// cell), however many those are, so that the host need not wait between
+/// rounds.
+__global__ void __launch_bounds__(128)
+k_dual_round(const __grid_constant__ DualArgs A, const DualTask* in, const uint32_t* n_in)
+{
+    const uint32_t n = n_in ? min(*n_in, A.out_cap) : 1u;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        DualTask task{};   // the root cell
+        if (n_in) task = in[t];
+        dual_task(A, task);
+    }
+}
+
 ////////////////////////////////////////////////////////////////////////////////
 // Small helpers for the host driver
 
@@ -2435,37 +2446,69 @@ __global__ void k_leaf_order_keys(const TapeRef* group_tape, uint32_t n,
     vals[i] = i;
 }
 
-__global__ void k_init_root(Octree o)
+/// What the kernels of one mesh count on the device, read back as a whole.
+struct MeshCounters {
+    uint32_t status;
+    uint32_t n_recs;
+    unsigned long long arena_top;
+    unsigned long long evals[2];
+    unsigned long long edge_top;
+    // zeroed before every octree level
+    unsigned long long list_top;
+    uint32_t next_cell;
+    uint32_t n_groups;       // branch cells of the level
+    uint32_t nregs;          // largest register count of their tapes
+    uint32_t pad;
+    // leaf stage
+    uint32_t next_group, next_group2;
+    uint32_t zero_top, n_redo;
+    uint32_t next_redo[2];
+    // dual walk
+    uint32_t n_tris;
+    uint32_t n_verts;
+    uint32_t n_tasks[kMaxLevels + 8];   // by round
+};
+constexpr size_t kLevelCounters = offsetof(MeshCounters, next_group) - offsetof(MeshCounters, list_top);
+
+__global__ void k_init_root(Octree o, MeshCounters* c, uint32_t n_clauses)
 {
     o.lv[0].coords[0] = 0;
+    o.lv[0].rec[0] = -1;
+    o.lv[0].child_group[0] = -1;
+    c->arena_top = n_clauses;
 }
 
-__global__ void k_branch_flags(const uint8_t* type, uint32_t n, uint32_t* flags)
+/// Flags of the branch cells (flags[n] = 0), how many there are and the
+/// largest register count of their tapes (which sizes the group-mode
+/// interval kernel's shared memory for the next depth).
+__global__ void k_branch_flags(const uint8_t* type, const TapeRef* cell_tape, uint32_t n,
+                               uint32_t* flags, MeshCounters* c)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flags[i] = type[i] == CELL_BRANCH ? 1u : 0u;
+    const bool branch = i < n && type[i] == CELL_BRANCH;
+    if (i <= n) flags[i] = branch ? 1u : 0u;
+    const uint32_t count = __popc(__ballot_sync(0xffffffffu, branch));
+    const uint32_t most = __reduce_max_sync(0xffffffffu, branch ? cell_tape[i].nregs : 0u);
+    if ((threadIdx.x & 31) == 0 && count) {
+        atomicAdd(&c->n_groups, count);
+        atomicMax(&c->nregs, most);
+    }
 }
 
 /// For each branch cell at depth d: its group index at d + 1, and the
 /// group's parent, tapes and child coordinates.
-__global__ void k_build_groups(Octree o, int d, const uint32_t* scan, uint32_t* nregs_next)
+__global__ void k_build_groups(Octree o, int d, const uint32_t* scan)
 {
     const LevelView& lv = o.lv[d];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool branch = i < lv.n_cells && lv.type[i] == CELL_BRANCH;
-    // largest register count of the next depth's group tapes (sizes the
-    // group-mode interval kernel's shared memory for that depth)
-    const uint32_t nr = branch ? lv.cell_tape[i].nregs : 0u;
-    const uint32_t wmax = __reduce_max_sync(0xffffffffu, nr);
-    if ((threadIdx.x & 31) == 0 && wmax) atomicMax(nregs_next, wmax);
     if (i >= lv.n_cells) return;
-    if (!branch) {
+    if (lv.type[i] != CELL_BRANCH) {
         lv.child_group[i] = -1;
         return;
     }
     const uint32_t g = scan[i];
     lv.child_group[i] = static_cast<int32_t>(g);
-    LevelView& nv = o.lv[d + 1];
+    const LevelView& nv = o.lv[d + 1];
     nv.group_parent[g] = i;
     nv.group_tape[g] = lv.cell_tape[i];
     nv.group_list[g] = lv.cell_list[i];
@@ -2474,6 +2517,7 @@ __global__ void k_build_groups(Octree o, int d, const uint32_t* scan, uint32_t* 
     for (int k = 0; k < 8; ++k) {
         nv.coords[8 * g + k] = pack_coords(2 * x + (k & 1), 2 * y + ((k >> 1) & 1),
                                            2 * z + ((k >> 2) & 1));
+        nv.rec[8 * g + k] = -1;
     }
 }
 
@@ -2580,6 +2624,7 @@ struct Workspace {
     std::map<int, DevBuf> bufs;
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
+    MeshCounters* seen = nullptr;   // page-locked: the counters as last read
     // Leaf edge records per leaf group (grows when a mesh needs more; the
     // mesh is then rendered again).
     uint32_t edges_per_group = 16;
@@ -2639,12 +2684,12 @@ Workspace* stream_workspace(unsigned k)
 }
 
 enum BufKey {
-    K_ARENA = 1, K_STATUS, K_COUNTERS, K_RECS, K_FLAGS, K_SCAN,
+    K_ARENA = 1, K_COUNTERS, K_RECS, K_FLAGS, K_SCAN,
     K_CUBTMP, K_TASK_A, K_TASK_B, K_TRIS, K_USED, K_VSCAN, K_VERTS, K_FEAT,
     K_LIST_A, K_LIST_B, K_WIDE_S, K_WIDE_SN, K_WIDE_P, K_WIDE_LIVE, K_WIDE_NEW,
     K_WIDE_ST2, K_WIDE_L1, K_WIDE_WL, K_LEAF_RD, K_ORDER_K0, K_ORDER_K1,
     K_ORDER_V0, K_ORDER_V1, K_SORTTMP, K_GDEC, K_GLAST, K_FEATWS,
-    K_EDGES, K_GEDGES, K_RECGROUP, K_NREGS, K_STL, K_COORDS, K_ZEROS, K_REDO,
+    K_EDGES, K_GEDGES, K_RECGROUP, K_STL, K_COORDS, K_ZEROS, K_REDO,
     K_VOPS, K_NSTEPS, K_ROOTTAPE,
     K_LEVEL = 100,
 };
@@ -2855,7 +2900,10 @@ namespace {
 /// Device -> pageable host copy: one transfer into a pinned staging buffer
 /// (grow-only, kept between calls), then a host copy split over a few
 /// threads (a single thread's memcpy is the slow part of a mesh download).
-bool download(Workspace& ws, void* dst, const void* src, size_t bytes, cudaStream_t s)
+/// wait = false: the caller waits for the stream when the destination is
+/// page-locked.
+bool download(Workspace& ws, void* dst, const void* src, size_t bytes, cudaStream_t s,
+              bool wait = true)
 {
     if (bytes == 0) return true;
     bool page_locked = false;
@@ -2867,7 +2915,7 @@ bool download(Workspace& ws, void* dst, const void* src, size_t bytes, cudaStrea
     if (page_locked) {
         // Page-locked destination: one direct transfer.
         return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "download") &&
-               cuda_ok(cudaStreamSynchronize(s), "download");
+               (!wait || cuda_ok(cudaStreamSynchronize(s), "download"));
     }
     void*& pinned = ws.pinned;
     if (bytes > ws.pinned_bytes) {
@@ -3020,16 +3068,26 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         return set_error(LFB_E_UNSUPPORTED, "tape needs more than 400 registers");
     }
 
-    uint32_t* status = ws.get<uint32_t>(K_STATUS, 1);
-    unsigned long long* counters = ws.get<unsigned long long>(K_COUNTERS, 10);
-    if (!status || !counters) return LFB_E_CUDA;
-    cudaMemsetAsync(status, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(counters, 0, 10 * sizeof(unsigned long long), s);
-    unsigned long long* edge_top = counters + 8;
-    unsigned long long* arena_top = counters + 1;
-    uint32_t* rec_top = reinterpret_cast<uint32_t*>(counters + 2);
-    unsigned long long* evals = counters + 3;
-    unsigned long long* list_top = counters + 5;
+    MeshCounters* counters = ws.get<MeshCounters>(K_COUNTERS, 1);
+    if (!counters) return LFB_E_CUDA;
+    if (!ws.seen && !cuda_ok(cudaMallocHost(reinterpret_cast<void**>(&ws.seen), sizeof(MeshCounters)),
+                             "page-locked counters")) {
+        return LFB_E_CUDA;
+    }
+    MeshCounters& seen = *ws.seen;
+    cudaMemsetAsync(counters, 0, sizeof(MeshCounters), s);
+    uint32_t* status = &counters->status;
+    unsigned long long* edge_top = &counters->edge_top;
+    unsigned long long* arena_top = &counters->arena_top;
+    uint32_t* rec_top = &counters->n_recs;
+    unsigned long long* evals = counters->evals;
+    unsigned long long* list_top = &counters->list_top;
+    // Reads the counters back; the host waits for them only where it has to
+    // know them to go on.
+    auto fetch_counters = [&](const char* what) {
+        return cuda_ok(cudaMemcpyAsync(&seen, counters, sizeof(MeshCounters), cudaMemcpyDeviceToHost, s),
+                       what);
+    };
     if (!g.ensure_wide()) return LFB_E_UNSUPPORTED;
 
     // Register-tape arena: the unpruned tape first, pruned tapes appended
@@ -3048,9 +3106,6 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
                                          cudaMemcpyDeviceToDevice, s), "arena")) {
         return LFB_E_CUDA;
     }
-    unsigned long long top_host = bt.n;
-    cudaMemcpyAsync(arena_top, &top_host, sizeof(top_host), cudaMemcpyHostToDevice, s);
-
     auto alloc_level = [&](int d, uint32_t n_cells, uint32_t n_groups) -> bool {
         LevelView& lv = o.lv[d];
         lv.n_cells = n_cells;
@@ -3069,12 +3124,11 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             !lv.group_parent || !lv.group_tape || !lv.cell_list || !lv.group_list) {
             return false;
         }
-        cudaMemsetAsync(lv.rec, 0xff, n_cells * sizeof(int32_t), s);
         return true;
     };
     // Level 0: the root cell.
     if (!alloc_level(0, 1, 0)) return LFB_E_CUDA;
-    k_init_root<<<1, 1, 0, s>>>(o);
+    k_init_root<<<1, 1, 0, s>>>(o, counters, bt.n);
     if (L == 0) {
         // No interval pass: the root is evaluated as a leaf right away.
         cudaMemsetAsync(o.lv[0].type, CELL_BRANCH, 1, s);
@@ -3109,10 +3163,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
     uint32_t* wL1 = ws.get<uint32_t>(K_WIDE_L1, scratch_warps * nw1);
     uint32_t* wWl = ws.get<uint32_t>(K_WIDE_WL, scratch_warps * nw16);
     if (!wS || !wSN || !wP || !wLive || !wNew || !wSt2 || !wL1 || !wWl) return LFB_E_CUDA;
-    if (L > 0) {
-        cudaMemsetAsync(wSt2, 0, scratch_warps * nw16 * 4, s);
-        cudaMemsetAsync(wL1, 0, scratch_warps * nw1 * 4, s);
-    }
+    bool wide_zeroed = false;   // the state words, which k_interval_wide leaves zero
     // Two list arenas, one per parity of depth: depth d reads the lists of
     // its groups from one and writes its children's lists to the other.
     const int list_key[2] = {K_LIST_A, K_LIST_B};
@@ -3129,10 +3180,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
     const uint32_t gdec_cap = std::max<uint32_t>(bt.n_choices, 1);
     uint8_t* gdec = ws.get<uint8_t>(K_GDEC, static_cast<size_t>(group_warps) * 8 * gdec_cap);
     uint8_t* glast = ws.get<uint8_t>(K_GLAST, static_cast<size_t>(group_warps) * 8 * kRenumberMax);
-    // per depth: the largest register count of its group tapes
-    uint32_t* level_nregs = ws.get<uint32_t>(K_NREGS, kMaxLevels + 2);
-    if (!gdec || !glast || !level_nregs) return LFB_E_CUDA;
-    cudaMemsetAsync(level_nregs, 0, (kMaxLevels + 2) * sizeof(uint32_t), s);
+    if (!gdec || !glast) return LFB_E_CUDA;
     bool group_mode = false;
     unsigned long long arena_used = bt.n;   // clauses in the arena
 
@@ -3141,17 +3189,12 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         LevelView& lv = o.lv[d];
         cells_evaluated += lv.n_cells;
         const auto t_level = std::chrono::steady_clock::now();
-        unsigned long long arena_before = 0;
-        uint32_t nregs_d = bt.n_regs;
-        cudaMemcpyAsync(&arena_before, arena_top, sizeof(arena_before), cudaMemcpyDeviceToHost, s);
-        if (d > 0) {
-            cudaMemcpyAsync(&nregs_d, level_nregs + d, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        }
-        if (!cuda_ok(cudaStreamSynchronize(s), "interval stage")) return LFB_E_CUDA;
+        const unsigned long long arena_before = arena_used;
         // The group-mode register file holds this depth's largest tape (the
         // pruned tapes of deep levels need far fewer registers than the
         // unpruned tape, so more warps fit on an SM).
-        nregs_d = std::min<uint32_t>(std::max<uint32_t>(nregs_d, 3), bt.n_regs);
+        const uint32_t nregs_d =
+            d == 0 ? bt.n_regs : std::min<uint32_t>(std::max<uint32_t>(seen.nregs, 3), bt.n_regs);
         const size_t group_smem = group_smem_per_warp(nregs_d) * 4;
         group_mode = group_mode || (d > 0 && lv.n_cells >= group_mode_cells() &&
                                     group_smem <= 200 * 1024);
@@ -3161,6 +3204,9 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         }
         const bool write_lists = d + 1 < L && !group_mode;
         const int out_key = list_key[(d + 1) & 1];
+        uint32_t* flags = ws.get<uint32_t>(K_FLAGS, lv.n_cells + 1);
+        uint32_t* scan = ws.get<uint32_t>(K_SCAN, lv.n_cells + 1);
+        if (!flags || !scan) return LFB_E_CUDA;
         for (int attempt = 0; attempt < 4; ++attempt) {
             WideArgs W;
             W.o = o;
@@ -3184,10 +3230,14 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             W.l1 = wL1;
             W.wl = wWl;
             W.status = status;
-            W.next_cell = reinterpret_cast<uint32_t*>(counters + 6);
+            W.next_cell = &counters->next_cell;
             W.group_shift = 3;
-            cudaMemsetAsync(W.next_cell, 0, sizeof(uint32_t), s);
-            cudaMemsetAsync(list_top, 0, sizeof(unsigned long long), s);
+            cudaMemsetAsync(list_top, 0, kLevelCounters, s);
+            if (!group_mode && lv.n_cells > block_mode_cells() && !wide_zeroed) {
+                wide_zeroed = true;
+                cudaMemsetAsync(wSt2, 0, scratch_warps * nw16 * 4, s);
+                cudaMemsetAsync(wL1, 0, scratch_warps * nw1 * 4, s);
+            }
             if (group_mode) {
                 GroupArgs G{o, bt, arena, arena_top, arena_cap, gdec, gdec_cap, glast,
                             nregs_d, status, W.next_cell};
@@ -3199,12 +3249,17 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             }
             ++n_launch;
             if (!cuda_ok(cudaGetLastError(), "interval kernel")) return LFB_E_CUDA;
-            uint32_t st = 0;
-            unsigned long long tops[2] = {0, 0};
-            cudaMemcpyAsync(&st, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(&tops[0], arena_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(&tops[1], list_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-            if (!cuda_ok(cudaStreamSynchronize(s), "interval kernel")) return LFB_E_CUDA;
+            // The level's counts go back while the branch cells are scanned:
+            // one wait per level.
+            k_branch_flags<<<lv.n_cells / 256 + 1, 256, 0, s>>>(lv.type, lv.cell_tape, lv.n_cells,
+                                                                flags, counters);
+            ++n_launch;
+            if (!fetch_counters("interval kernel") || !exclusive_scan(ws, flags, scan, lv.n_cells + 1, s) ||
+                !cuda_ok(cudaStreamSynchronize(s), "interval kernel")) {
+                return LFB_E_CUDA;
+            }
+            const uint32_t st = seen.status;
+            const unsigned long long tops[2] = {seen.arena_top, seen.list_top};
             if (st & ST_REGS) {
                 return set_error(LFB_E_UNSUPPORTED, "tape register renumbering failed");
             }
@@ -3258,21 +3313,13 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
                          d, lv.n_cells, top_now, lt, ms);
         }
         // Compact the branch cells into the groups of depth d + 1.
-        uint32_t* flags = ws.get<uint32_t>(K_FLAGS, lv.n_cells + 1);
-        uint32_t* scan = ws.get<uint32_t>(K_SCAN, lv.n_cells + 1);
-        if (!flags || !scan) return LFB_E_CUDA;
-        k_branch_flags<<<(lv.n_cells + 255) / 256, 256, 0, s>>>(lv.type, lv.n_cells, flags);
-        cudaMemsetAsync(flags + lv.n_cells, 0, sizeof(uint32_t), s);
-        if (!exclusive_scan(ws, flags, scan, lv.n_cells + 1, s)) return LFB_E_CUDA;
-        uint32_t n_groups = 0;
-        cudaMemcpyAsync(&n_groups, scan + lv.n_cells, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        if (!cuda_ok(cudaStreamSynchronize(s), "scan")) return LFB_E_CUDA;
+        const uint32_t n_groups = seen.n_groups;
         if (static_cast<uint64_t>(n_groups) * 8 >= (1u << 27)) {
             return set_error(LFB_E_CAPACITY, "more than 2^27 cells on one octree level");
         }
         if (!alloc_level(d + 1, n_groups * 8, n_groups)) return LFB_E_CUDA;
-        k_build_groups<<<(lv.n_cells + 255) / 256, 256, 0, s>>>(o, d, scan, level_nregs + d + 1);
-        n_launch += 2;   // k_branch_flags + k_build_groups
+        k_build_groups<<<(lv.n_cells + 255) / 256, 256, 0, s>>>(o, d, scan);
+        ++n_launch;
         if (n_groups == 0) {
             // Nothing ambiguous below this depth: no leaves, no faces.
             o.levels = L;
@@ -3348,11 +3395,10 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         if (!scratch) return LFB_E_CUDA;
         float* rd = ws.get<float>(K_LEAF_RD, slices * bt.n_regs * 128);
         if (!rd) return LFB_E_CUDA;
-        uint32_t* next_group = reinterpret_cast<uint32_t*>(counters + 7);
-        cudaMemsetAsync(next_group, 0, sizeof(uint32_t), s);
-        // Longest tapes first.
+        uint32_t* next_group = &counters->next_group;
+        // Longest tapes first, where not all groups run at once anyway.
         const uint32_t* order = nullptr;
-        if (L > 0 && n_leaf_groups > 1) {
+        if (L > 0 && n_leaf_groups > grid * wpb) {
             uint32_t* k0 = ws.get<uint32_t>(K_ORDER_K0, n_leaf_groups);
             uint32_t* k1 = ws.get<uint32_t>(K_ORDER_K1, n_leaf_groups);
             uint32_t* v0 = ws.get<uint32_t>(K_ORDER_V0, n_leaf_groups);
@@ -3362,12 +3408,14 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
                 o.lv[L].group_tape, n_leaf_groups, k0, v0);
             ++n_launch;
             size_t tmp = 0;
+            int bits = 1;   // of a tape length
+            while (bits < 32 && (bt.n >> bits)) ++bits;
             cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, k0, k1, v0, v1,
-                                                      static_cast<int>(n_leaf_groups), 0, 32, s);
+                                                      static_cast<int>(n_leaf_groups), 0, bits, s);
             void* t = ws.get<unsigned char>(K_SORTTMP, tmp);
             if (!t || !cuda_ok(cub::DeviceRadixSort::SortPairsDescending(
                                    t, tmp, k0, k1, v0, v1, static_cast<int>(n_leaf_groups), 0,
-                                   32, s), "leaf order")) {
+                                   bits, s), "leaf order")) {
                 return LFB_E_CUDA;
             }
             order = v1;
@@ -3381,7 +3429,6 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         GroupEdges* gedges = ws.get<GroupEdges>(K_GEDGES, n_leaf_groups);
         uint32_t* rec_group = ws.get<uint32_t>(K_RECGROUP, rec_cap);
         if (!edges || !gedges || !rec_group) return LFB_E_CUDA;
-        cudaMemsetAsync(rec_group, 0xff, rec_cap * sizeof(uint32_t), s);
         // Steps by clause offset, so room for as many as the arena has clauses.
         ValOp* vops = ws.get<ValOp>(K_VOPS, arena_used);
         uint32_t* n_steps = ws.get<uint32_t>(K_NSTEPS, arena_used);
@@ -3392,16 +3439,15 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         const uint32_t zero_cap = small ? 0u : static_cast<uint32_t>(std::min<uint64_t>(
             static_cast<uint64_t>(n_leaf_groups) * 32 + 4096, 1u << 30));
         float* zeros = ws.get<float>(K_ZEROS, size_t{3} * zero_cap);
-        uint32_t* redo = ws.get<uint32_t>(K_REDO, size_t{2} * n_leaf_groups + 4);
+        uint32_t* redo = ws.get<uint32_t>(K_REDO, n_leaf_groups);
         if (!zeros || !redo) return LFB_E_CUDA;
-        uint32_t* redo_counts = redo + 2 * static_cast<size_t>(n_leaf_groups);
-        cudaMemsetAsync(redo_counts, 0, 4 * sizeof(uint32_t), s);
         LeafArgs A{o, bt, arena, recs, rec_top, static_cast<uint32_t>(rec_cap), status,
                    evals, scratch, rd, group_regs, next_group, order, featws,
                    edges, edge_top, edge_cap, gedges, rec_group,
-                   reinterpret_cast<uint32_t*>(counters + 9),
+                   &counters->next_group2,
                    vops, n_steps, n_leaf_groups >= kLeafChunk * 4 * grid * wpb ? kLeafChunk : 1u,
-                   zeros, redo_counts, zero_cap, redo, redo_counts + 1, redo_counts + 2};
+                   zeros, &counters->zero_top, zero_cap, redo, &counters->n_redo,
+                   counters->next_redo};
         const TapeRef* tapes = o.lv[L].group_tape;
         if (L == 0) {
             // the unpruned tape is the only one
@@ -3476,17 +3522,19 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
     }
 
     if (stats) cudaEventRecord(ev[3], s);
-    uint32_t st = 0, n_recs = 0;
-    cudaMemcpyAsync(&st, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&n_recs, rec_top, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (!cuda_ok(cudaStreamSynchronize(s), "leaf/collapse")) return LFB_E_CUDA;
+    if (!fetch_counters("leaf/collapse") ||
+        !cuda_ok(cudaMemcpyAsync(&seen.pad, o.lv[0].type, 1, cudaMemcpyDeviceToHost, s),
+                 "leaf/collapse") ||
+        !cuda_ok(cudaStreamSynchronize(s), "leaf/collapse")) {
+        return LFB_E_CUDA;
+    }
+    const uint8_t root_type = static_cast<uint8_t>(seen.pad & 0xff);
+    const uint32_t st = seen.status, n_recs = seen.n_recs;
     if (st & ST_RECORD_OVERFLOW) return set_error(LFB_E_CAPACITY, "leaf record overflow");
     if (st & ST_EDGE_OVERFLOW) {
         // more crossing edges than records were reserved for: grow, and the
         // caller renders the mesh again
-        unsigned long long need = 0;
-        cudaMemcpyAsync(&need, edge_top, sizeof(need), cudaMemcpyDeviceToHost, s);
-        cudaStreamSynchronize(s);
+        const unsigned long long need = seen.edge_top;
         const uint32_t groups = std::max<uint32_t>(n_leaf_groups, 1);
         ws.edges_per_group = static_cast<uint32_t>(std::min<unsigned long long>(
             54, need / groups + 2));
@@ -3517,9 +3565,6 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
     out.tri_count = 0;
     if (!out.verts) return set_error(LFB_E_CAPACITY, "host allocation failed");
     out.verts[0] = {0.0f, 0.0f, 0.0f};
-    uint8_t root_type = 0;
-    cudaMemcpyAsync(&root_type, o.lv[0].type, 1, cudaMemcpyDeviceToHost, s);
-    cudaStreamSynchronize(s);
     const uint32_t n_keys = n_recs * 4;
     bool stl_written = false;
     if (root_type == CELL_BRANCH && n_recs) {
@@ -3532,49 +3577,43 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             uint8_t* used = ws.get<uint8_t>(K_USED, n_keys + 1);
             if (!qa || !qb || !tris || !used) return LFB_E_CUDA;
             cudaMemsetAsync(used, 0, n_keys + 1, s);
-            uint32_t* n_out = reinterpret_cast<uint32_t*>(counters + 5);
-            uint32_t* n_tris = reinterpret_cast<uint32_t*>(counters + 6);
-            cudaMemsetAsync(n_tris, 0, sizeof(uint32_t), s);
+            cudaMemsetAsync(&counters->n_tris, 0, sizeof(MeshCounters) - offsetof(MeshCounters, n_tris), s);
             cudaMemsetAsync(status, 0, sizeof(uint32_t), s);
-            DualTask root{};
-            root.kind = TASK_CELL;
-            cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, s);
-            uint32_t n_in = 1;
-            DualArgs D{o, recs, status, qb, n_out, static_cast<uint32_t>(task_cap),
-                       tris, n_tris, static_cast<uint32_t>(tri_cap), used};
-            bool overflow = false;
-            while (n_in) {
+            DualArgs D{o, recs, status, qb, nullptr, static_cast<uint32_t>(task_cap),
+                       tris, &counters->n_tris, static_cast<uint32_t>(tri_cap), used};
+            // A task's cells are one depth deeper every round, so L + 2
+            // rounds leave none; each reads how many tasks there are itself.
+            const uint32_t dual_blocks = std::min<uint32_t>(
+                static_cast<uint32_t>(device_sm_count()) * 32, n_recs / 16 + 1);
+            for (int r = 0; r < L + 2; ++r) {
                 if (cancelled()) return LFB_E_CANCELLED;
-                cudaMemsetAsync(n_out, 0, sizeof(uint32_t), s);
                 D.out = qb;
-                k_dual_round<<<(n_in + 127) / 128, 128, 0, s>>>(D, qa, n_in);
+                D.n_out = counters->n_tasks + r;
+                k_dual_round<<<r == 0 ? 1 : dual_blocks, 128, 0, s>>>(
+                    D, qa, r == 0 ? nullptr : counters->n_tasks + r - 1);
                 ++n_launch;
-                uint32_t st2 = 0;
-                cudaMemcpyAsync(&n_in, n_out, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-                cudaMemcpyAsync(&st2, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-                if (!cuda_ok(cudaStreamSynchronize(s), "dual walk")) return LFB_E_CUDA;
-                if (st2 & ST_QUEUE_OVERFLOW) {
-                    overflow = true;
-                    break;
-                }
                 std::swap(qa, qb);
             }
-            if (overflow) {
-                task_cap *= 4;
-                tri_cap *= 4;
-                continue;
-            }
-            uint32_t n_tri = 0;
-            cudaMemcpyAsync(&n_tri, n_tris, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
             // Vertex numbering: ids in record order, 0 is the placeholder.
             uint32_t* flags = ws.get<uint32_t>(K_FLAGS, n_keys + 1);
             uint32_t* vscan = ws.get<uint32_t>(K_VSCAN, n_keys + 1);
             if (!flags || !vscan) return LFB_E_CUDA;
             k_u8_to_u32<<<(n_keys + 1 + 255) / 256, 256, 0, s>>>(used, flags, n_keys + 1);
-            if (!exclusive_scan(ws, flags, vscan, n_keys + 1, s)) return LFB_E_CUDA;
-            uint32_t n_verts = 0;
-            cudaMemcpyAsync(&n_verts, vscan + n_keys, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-            if (!cuda_ok(cudaStreamSynchronize(s), "vertex scan")) return LFB_E_CUDA;
+            if (!exclusive_scan(ws, flags, vscan, n_keys + 1, s) || !fetch_counters("dual walk") ||
+                !cuda_ok(cudaMemcpyAsync(&seen.n_verts, vscan + n_keys, sizeof(uint32_t),
+                                         cudaMemcpyDeviceToHost, s), "dual walk") ||
+                !cuda_ok(cudaStreamSynchronize(s), "dual walk")) {
+                return LFB_E_CUDA;
+            }
+            if (seen.status & ST_QUEUE_OVERFLOW) {
+                task_cap *= 4;
+                tri_cap *= 4;
+                continue;
+            }
+            const uint32_t n_tri = seen.n_tris, n_verts = seen.n_verts;
+            if (seen.n_tasks[L + 1] != 0) {   // cannot happen
+                return set_error(LFB_E_CAPACITY, "dual walk did not end");
+            }
             float* verts = ws.get<float>(K_VERTS, 3 * (static_cast<size_t>(n_verts) + 1));
             if (!verts) return LFB_E_CUDA;
             cudaMemsetAsync(verts, 0, 3 * sizeof(float), s);
@@ -3598,28 +3637,31 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             if (!out.verts) return set_error(LFB_E_CAPACITY, "host allocation failed");
             out.vert_count = n_verts + 1;
             out.tri_count = n_tri;
-            if (!download(ws, out.verts, verts, out.vert_count * sizeof(libfive_vec3), s)) {
-                return LFB_E_CUDA;
-            }
-            if (out.format == MeshFormat::Coords) {
-                int4* c = ws.get<int4>(K_COORDS, std::max<uint32_t>(n_tri, 1));
+            const bool coords = out.format == MeshFormat::Coords;
+            int4* c = nullptr;
+            if (coords) {
+                c = ws.get<int4>(K_COORDS, std::max<uint32_t>(n_tri, 1));
                 host_free(out.coords);
                 out.coords = static_cast<int32_t*>(host_alloc(static_cast<size_t>(n_tri) * 16));
                 if (!c) return LFB_E_CUDA;
-                if (!out.coords && n_tri) return set_error(LFB_E_CAPACITY, "host allocation failed");
-                if (n_tri) {
-                    k_pack_coords<<<(n_tri + 255) / 256, 256, 0, s>>>(tris, n_tri, c);
-                    ++n_launch;
-                    if (!download(ws, out.coords, c, static_cast<size_t>(n_tri) * 16, s)) {
-                        return LFB_E_CUDA;
-                    }
-                }
-                break;
+            } else {
+                out.tris = static_cast<libfive_tri*>(
+                    host_alloc(static_cast<size_t>(n_tri) * sizeof(libfive_tri)));
             }
-            out.tris = static_cast<libfive_tri*>(
-                host_alloc(static_cast<size_t>(n_tri) * sizeof(libfive_tri)));
-            if (!out.tris) return set_error(LFB_E_CAPACITY, "host allocation failed");
-            if (!download(ws, out.tris, tris, static_cast<size_t>(n_tri) * sizeof(libfive_tri), s)) {
+            if (coords ? !out.coords && n_tri : !out.tris) {
+                return set_error(LFB_E_CAPACITY, "host allocation failed");
+            }
+            if (coords && n_tri) {
+                k_pack_coords<<<(n_tri + 255) / 256, 256, 0, s>>>(tris, n_tri, c);
+                ++n_launch;
+            }
+            // one wait for both downloads, when there is a second
+            const bool ok =
+                download(ws, out.verts, verts, out.vert_count * sizeof(libfive_vec3), s, n_tri == 0) &&
+                (coords ? download(ws, out.coords, c, static_cast<size_t>(n_tri) * 16, s)
+                        : download(ws, out.tris, tris, static_cast<size_t>(n_tri) * sizeof(libfive_tri), s));
+            if (!ok) {
+                cudaStreamSynchronize(s);   // nothing may still be writing to the arrays
                 return LFB_E_CUDA;
             }
             break;
