@@ -48,6 +48,16 @@ int eval_grad(GpuTape& g, uint64_t n, const float* x, const float* y,
               float* gy, float* gz, float* gvars, cudaStream_t s,
               bool device);
 
+/// Floats of scratch that eval_grad_with needs for n points of the tape, or
+/// 0 when it does not take them (no checkpointed kernels, CONST_VAR, more
+/// points than one launch).
+uint64_t grad_scratch_floats(GpuTape& g, uint64_t n);
+/// f at n points and gvars += sum f df/dvar (eval_grad with seed f), device
+/// arrays, checkpoints in the caller's scratch: calls with scratch of their
+/// own may run at once on different streams.
+int eval_grad_with(GpuTape& g, uint64_t n, const float* x, const float* y, const float* z, float* f,
+                   float* gvars, float* scratch, cudaStream_t s);
+
 /// Builds what the reverse mode needs for this tape (partial-slot table,
 /// compiled partials and backward kernels) without launching anything, so
 /// that many tapes can be prepared on several host threads at once.

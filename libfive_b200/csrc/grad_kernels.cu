@@ -720,6 +720,25 @@ int eval_loss_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const
     return cuda_ok(cudaGetLastError(), "loss gradient") ? 0 : LFB_E_CUDA;
 }
 
+uint64_t grad_scratch_floats(GpuTape& g, uint64_t n)
+{
+    const uint32_t ckf = tape_has_const_var(g) ? 0 : jit_ckpt_prepare(g);
+    // one launch pair: no more points than grad_device takes at once
+    return ckf && n <= (uint64_t(1) << 22) ? n * ckf : 0;
+}
+
+int eval_grad_with(GpuTape& g, uint64_t n, const float* x, const float* y, const float* z, float* f,
+                   float* gvars, float* scratch, cudaStream_t s)
+{
+    const uint32_t m = static_cast<uint32_t>(n);
+    if (!jit_ckpt_forward(g, m, x, y, z, scratch, f, s) ||
+        (gvars && !jit_ckpt_backward(g, m, scratch, f, nullptr, nullptr, nullptr, gvars, 0, s)) ||
+        !cuda_ok(cudaGetLastError(), "gradient kernels")) {
+        return set_error(LFB_E_CUDA, "checkpointed gradient kernel launch failed");
+    }
+    return 0;
+}
+
 int eval_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const float* z,
               const float* seed, float* f, float* gx, float* gy, float* gz, float* gvars,
               cudaStream_t s, bool device)
