@@ -829,12 +829,16 @@ std::string ckpt_backward_source(const RegTape& t)
          "    const unsigned k = lfb_vidx[base + lane];\n"
          "    if (k != 0xffffu && v[0] != 0.0f) atomicAdd(Gv + k, v[0]);\n}\n";
     s += body;
-    // at most 64 registers a thread: four blocks of 256 threads on an SM.
+    // Blocks of 256 threads on an SM: three (80 registers a thread) for
+    // tapes of three or more segments, four (64) for shorter ones.  1,017
+    // clauses, 10^6 points: loss and gradient 838 us with four, 771 with
+    // three, 899 with two; six 377-clause shapes of 65,536 points 166 us with
+    // four, 168 with three.
     // (One 1024-thread block with a barrier before each segment, so that
     // an SM's warps share a segment's instruction fetches, was measured
     // slower: the barriers cost more than the fetch stalls they saved.)
     s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(kCkptBwdBlock) +
-         ", 4)\n"
+         (segs.size() >= 3 ? ", 3)\n" : ", 4)\n") +
          "lfb_tape_ckpt_bwd(const float* __restrict__ C, const float* __restrict__ seed,\n"
          "                  float* __restrict__ gx, float* __restrict__ gy,\n"
          "                  float* __restrict__ gz, float* __restrict__ gvars, unsigned m,\n"
