@@ -93,9 +93,11 @@ __device__ __forceinline__ WideConsts wide_consts(const uint4& e, const float* _
 
 /// Interval of list entry k, stored in slot 3 + k, and the entry's state for
 /// the cell's children; returns whether a min/max got decided
-/// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167).
+/// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167); nan_safe:
+/// not between operands that may be NaN.
 __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c, uint32_t k,
-                                             float2* S, uint8_t* SN, uint8_t* pst)
+                                             float2* S, uint8_t* SN, uint8_t* pst,
+                                             bool nan_safe = false)
 {
     const uint8_t o = e.x & 0xff;
     const uint32_t kinds = (e.x >> 8) & 0xf;
@@ -115,7 +117,7 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
             uint8_t keep = 0;   // 0 both, 1 a, 2 b
             if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;
             else if (b.lo > a.hi) keep = (o == op::MAX) ? 2 : 1;
-            if (keep) {
+            if (keep && !(nan_safe && (a.nan || b.nan))) {
                 ps = keep == 1 ? WIDE_A : WIDE_B;
                 decided = true;
             }
@@ -569,6 +571,8 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
     const Octree& o = A.o;
     const LevelView& lv = o.lv[d];
     const DevTape& bt = A.bt;
+    const bool boxes = A.boxes != nullptr;
+    const uint32_t n_cells = boxes ? A.n_boxes : lv.n_cells;
     const uint32_t n = A.n;
     const size_t slot = blockIdx.x;
 
@@ -577,10 +581,10 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
         __syncthreads();
         const uint32_t i = cell;
         __syncthreads();
-        if (i >= lv.n_cells) break;
+        if (i >= n_cells) break;
         ListRef P;
         TapeRef T;
-        if (d == 0) {
+        if (boxes || d == 0) {
             P = A.root_list;
             T = root_tape_ref(bt);
         } else {
@@ -622,9 +626,14 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
         uint4 e{}, e_next{};
         fetch(0, e);
         if (tid < 3) {
-            double blo[3], bhi[3];
-            cell_bounds(o, d, lv.coords[i], blo, bhi);
-            const Iv v = iv_make(static_cast<float>(blo[tid]), static_cast<float>(bhi[tid]));
+            Iv v;
+            if (boxes) {
+                v = iv_make(A.boxes[6 * i + 2 * tid], A.boxes[6 * i + 2 * tid + 1]);
+            } else {
+                double blo[3], bhi[3];
+                cell_bounds(o, d, lv.coords[i], blo, bhi);
+                v = iv_make(static_cast<float>(blo[tid]), static_cast<float>(bhi[tid]));
+            }
             S[tid] = make_float2(v.lo, v.hi);
             SN[tid] = v.nan;
         }
@@ -642,7 +651,7 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
             fetch(w + 1, e_next);
             c_next = wide_consts(e_next, bt.cpool);
             for (uint32_t l = lf; l <= ll; ++l) {
-                if (lev == l) changed |= wide_forward(e, c, k, S, SN, pst);
+                if (lev == l) changed |= wide_forward(e, c, k, S, SN, pst, boxes);
                 __syncthreads();
             }
             e = e_next;
@@ -652,13 +661,17 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
         const float root_c = bt.root_kind == OPND_REG ? 0.0f : __ldg(bt.cpool + P.root);
         const Iv root = wide_fetch(bt.root_kind, P.root, root_c, S, SN);
         const uint8_t state = iv_state(root);
-        if (tid == 0) {
+        if (tid == 0 && !boxes) {
             lv.type[i] = state == ST_EMPTY ? CELL_EMPTY
                        : state == ST_FILLED ? CELL_FILLED : CELL_BRANCH;
         }
-        if (state != ST_AMBIGUOUS) return;
+        if (!boxes && state != ST_AMBIGUOUS) return;
+        if (boxes && !changed) {
+            if (tid == 0) A.box_tape[i] = T;
+            return;
+        }
 
-        if (root.nan || !changed) {
+        if (!boxes && (root.nan || !changed)) {
             // The children keep this tape; its list moves to the next arena.
             uint32_t off = 0;
             if (A.write_lists) {
@@ -781,7 +794,7 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
         uint32_t pos = warp_counts_scan(emit, warp_tot, etot);
         if (tid == 0) bcast = atomicAdd(A.arena_top, static_cast<unsigned long long>(etot));
         __syncthreads();
-        const unsigned long long a64 = bcast;
+        const unsigned long long a64 = bcast + A.arena_base;
         const bool aok = a64 + etot <= A.arena_cap;
         if (!aok && tid == 0) atomicOr(A.status, ST_ARENA_OVERFLOW);
         uint2* to = reinterpret_cast<uint2*>(A.arena + a64);
@@ -797,7 +810,9 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
             out_t = {static_cast<uint32_t>(a64), etot, bt.n_regs,
                      static_cast<uint32_t>(bt.root) | (static_cast<uint32_t>(bt.root_kind) << 16)};
         }
-        if (tid == 0) {
+        if (tid == 0 && boxes) {
+            A.box_tape[i] = out_t;
+        } else if (tid == 0) {
             lv.cell_list[i] = {loff, cnt, new_root, 0u};
             lv.cell_tape[i] = out_t;
         }
@@ -2751,6 +2766,36 @@ bool debug_levels()
 
 }  // namespace
 
+namespace {
+
+/// Entries whose state fits the shared memory of a block when `per_sm`
+/// blocks share an SM, and the bytes that takes.
+uint32_t block_slots(uint32_t n, uint32_t per_sm)
+{
+    return std::min<uint32_t>((n + 3) / 4 * 4, (216u * 1024 / per_sm - 2048) / 11 / 4 * 4);
+}
+size_t block_smem(uint32_t slots) { return (11 * static_cast<size_t>(slots) + 27 + 15) / 16 * 16; }
+
+}  // namespace
+
+uint32_t interval_box_slots(uint32_t n, uint32_t n_boxes)
+{
+    // Two blocks an SM when a list's state then still fits, else one.
+    const uint32_t sms = static_cast<uint32_t>(device_sm_count());
+    return std::min(n_boxes, block_slots(n, 2) >= n ? 2 * sms : sms);
+}
+
+cudaError_t launch_interval_boxes(const WideArgs& W, uint32_t slots, cudaStream_t s)
+{
+    const uint32_t n_slots = block_slots(W.n, block_slots(W.n, 2) >= W.n ? 2 : 1);
+    const size_t smem = block_smem(n_slots);
+    if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_block), smem)) {
+        return cudaErrorInvalidValue;
+    }
+    k_interval_block<<<std::max<uint32_t>(slots, 1), kBlockThreads, smem, s>>>(W, 0, n_slots);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_interval_lists(const WideArgs& W, int d, uint32_t n_cells, uint32_t scratch_warps,
                                   cudaStream_t s)
 {
@@ -2760,8 +2805,8 @@ cudaError_t launch_interval_lists(const WideArgs& W, int d, uint32_t n_cells, ui
         // (their lists are pruned): two blocks then share an SM.
         const uint32_t sms = static_cast<uint32_t>(device_sm_count());
         const uint32_t per_sm = n_cells <= sms ? 1 : 2;
-        const uint32_t slots = std::min<uint32_t>((W.n + 3) / 4 * 4, (216u * 1024 / per_sm - 2048) / 11 / 4 * 4);
-        const size_t smem = (11 * static_cast<size_t>(slots) + 27 + 15) / 16 * 16;
+        const uint32_t slots = block_slots(W.n, per_sm);
+        const size_t smem = block_smem(slots);
         if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_block), smem)) {
             return cudaErrorInvalidValue;
         }
@@ -3232,6 +3277,9 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             W.status = status;
             W.next_cell = &counters->next_cell;
             W.group_shift = 3;
+            W.boxes = nullptr;
+            W.n_boxes = W.arena_base = 0;
+            W.box_tape = nullptr;
             cudaMemsetAsync(list_top, 0, kLevelCounters, s);
             if (!group_mode && lv.n_cells > block_mode_cells() && !wide_zeroed) {
                 wide_zeroed = true;

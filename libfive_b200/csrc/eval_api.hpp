@@ -43,6 +43,12 @@ int eval_loss_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const
                    float* f, float* gx, float* gy, float* gz, float* gvars, float* loss,
                    cudaStream_t s);
 
+/// Derivatives of a long tape by pruning it for cells of neighbouring
+/// points (pruned_derivs.cu; the interpreter's results); false when it does
+/// not take the call, which then has done nothing.
+bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const float* z, float* v,
+                   float* dx, float* dy, float* dz, cudaStream_t s);
+
 int eval_grad(GpuTape& g, uint64_t n, const float* x, const float* y,
               const float* z, const float* seed, float* f, float* gx,
               float* gy, float* gz, float* gvars, cudaStream_t s,

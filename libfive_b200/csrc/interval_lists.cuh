@@ -35,6 +35,14 @@ struct WideArgs {
     uint32_t* status;
     uint32_t* next_cell;           // work counter (zero at launch)
     uint32_t group_shift;          // cells per group: 8 (3) in an octree, 4 (2) in a quadtree
+    // Box form (launch_interval_boxes): the unpruned tape pruned for each of
+    // n_boxes boxes (lower and upper bound per axis), whatever the sign of its
+    // interval, min / max clauses decided only between operands that cannot
+    // be NaN.  The arena's tapes start after arena_base clauses.
+    const float* boxes;
+    uint32_t n_boxes;
+    uint32_t arena_base;
+    TapeRef* box_tape;
 };
 
 /// Bytes of WideArgs' per-warp scratch for `warps` warps over a tape of n
@@ -65,5 +73,10 @@ inline void wide_scratch_carve(WideArgs& W, unsigned char* p, uint64_t n, uint64
 /// cell for few cells, a warp a cell otherwise.
 cudaError_t launch_interval_lists(const WideArgs& W, int d, uint32_t n_cells, uint32_t scratch_warps,
                                   cudaStream_t s);
+
+/// The box form: scratch slots (blocks) that it wants for a tape of n
+/// clauses, and its launch.
+uint32_t interval_box_slots(uint32_t n, uint32_t n_boxes);
+cudaError_t launch_interval_boxes(const WideArgs& W, uint32_t slots, cudaStream_t s);
 
 }  // namespace lfb

@@ -47,6 +47,7 @@ struct GpuTape {
     uint32_t wide_root = 0;
     bool wide_ready = false;
     bool ensure_wide();
+    int sound_ops = -1;   // whether pruned_derivs takes its opcodes (-1: not looked at yet)
 
     // Reverse mode: where each clause's local partials are stored per point
     // (slot | kind << 28, see grad_kernels.cu), built on first use.
