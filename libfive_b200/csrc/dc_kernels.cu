@@ -5,20 +5,21 @@
 // the dual grid with another pool (Dual<3>::walk, dual.hpp:126-385).  Here
 // every stage is a level-synchronous pass over compacted arrays:
 //
-//   1. k_interval_level   (once per depth d < L)
+//   1. k_interval_block / _wide / _group   (one of them per depth d < L)
 //        DCTree::evalInterval (dc_tree.inl:94-128): interval-evaluate every
 //        cell of depth d with the tape of its parent, classify it
 //        EMPTY / FILLED / AMBIGUOUS, and prune the tape for its children
 //        (Tape::push, tape.cpp:23-160) as a backward liveness pass over the
 //        register tape; decided min/max clauses become register copies.
-//   2. k_leaf_groups      (depth L)
+//   2. k_leaf_decode, k_leaf_groups, k_leaf_qef, k_edge_rank,
+//      k_leaf_vertices    (depth L)
 //        DCTree::evalLeaf (dc_tree.inl:131-552) for the eight children of
 //        each ambiguous depth L-1 cell, one warp per sibling group: the 27
 //        shared corners, the crossing edges of the 3x3x3 lattice (each
 //        searched once), the QEFs and the per-patch vertices.
 //   3. k_collapse_level   (depths L-1 .. 0)
 //        DCTree::collectChildren (dc_tree.inl:581-735).
-//   4. k_dual_round       (until no task is left)
+//   4. k_dual_round       (one round per depth, launched without waiting)
 //        Dual<3>::work / face3 / edge3 as a breadth-first task expansion and
 //        DCMesher::load (dc_mesher.cpp:18-169) at minimal edges.
 //
@@ -1116,9 +1117,9 @@ __device__ __forceinline__ float4 dv_value4f(uint8_t o, const float4& a, const f
 /// Values of the tape at four points per lane (point k of this lane in
 /// component k) for tapes with more registers than the shared-memory file
 /// holds: the clauses are streamed (one fetched ahead), the register file R
-/// (x, y, z in its first three) is in global memory.  With ties, bit k of *amb reports a min / max with
-/// equal arguments at point k (ArrayEvaluator::getAmbiguous,
-/// eval_array.cpp:197-217).
+/// (x, y, z in its first three) is in global memory.  With ties, bit k of
+/// *amb reports a min / max with equal arguments at point k
+/// (ArrayEvaluator::getAmbiguous, eval_array.cpp:197-217).
 static __device__ __noinline__ float4 warp_value4(const float* __restrict__ cpool,
                                                   uint32_t root_kind, uint32_t root,
                                                   const RegClause* __restrict__ cl, uint32_t len,

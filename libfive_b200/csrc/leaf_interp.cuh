@@ -5,12 +5,13 @@
 // with derivatives (DerivArrayEvaluator::derivs, eval_deriv_array.cpp:
 // 101-117).
 //
-// Layout for throughput on an interpreter whose cost is per clause:
-//  * the warp first decodes a chunk of kLeafOps register-tape clauses into
-//    LeafOps in shared memory (one clause per lane): opcode and operand kinds
-//    become one handler number, constant and free-variable operands become
-//    an immediate value, so the evaluation loop reads one 16-byte broadcast
-//    word per clause and branches once;
+// Layout for throughput on an interpreter whose cost is per step:
+//  * clauses are decoded before they are run.  Values: k_leaf_decode turns a
+//    tape into fused steps once (ValOp, several clauses each) and a warp
+//    fetches them into shared memory.  Derivatives: the warp decodes
+//    kLeafOps clauses at a time into LeafOps in shared memory (one clause
+//    per lane), where opcode and operand kinds have become one handler
+//    number and a constant or free-variable operand an immediate value;
 //  * the register file holds one float4 per (register, lane): the four
 //    points of a lane (or value + gradient) move with one 128-bit shared
 //    memory access per operand.
@@ -168,9 +169,6 @@ __device__ __forceinline__ uint32_t leaf_decode_chunk(LeafOp* ops, const LeafRaw
 
 __device__ __forceinline__ float4 splat4(float v) { return make_float4(v, v, v, v); }
 
-#define LFB_MAP2(F, a, b) make_float4(F((a).x, (b).x), F((a).y, (b).y), F((a).z, (b).z), F((a).w, (b).w))
-#define LFB_MAP1(F, a) make_float4(F((a).x), F((a).y), F((a).z), F((a).w))
-
 __device__ __forceinline__ float f_square(float a) { return __fmul_rn(a, a); }
 __device__ __forceinline__ float f_neg(float a) { return -a; }
 __device__ __forceinline__ float f_sqrt(float a) { return __fsqrt_rn(a); }
@@ -191,9 +189,6 @@ static __device__ __noinline__ float4 leaf_generic4(uint8_t o, float4 a, float4 
     return make_float4(dv_value(o, a.x, b.x), dv_value(o, a.y, b.y), dv_value(o, a.z, b.z),
                        dv_value(o, a.w, b.w));
 }
-
-#undef LFB_MAP1
-#undef LFB_MAP2
 
 ////////////////////////////////////////////////////////////////////////////////
 // Values: fused steps
