@@ -260,12 +260,14 @@ int fit_adam_step(GpuTape* const* tapes, uint32_t n_shapes, const uint64_t* poff
         lane_floats = std::max(lane_floats, c);
         side_by_side = c != 0 && lane_floats * lanes <= kFitLaneFloats;
     }
-    side_by_side = side_by_side && sc.make_lanes();
+    if (side_by_side &&
+        !(sc.make_lanes() && sc.ckpt.reserve(lane_floats * lanes * sizeof(float)))) {
+        cudaGetLastError();   // one after another needs less
+        clear_error();
+        side_by_side = false;
+    }
     if (side_by_side) {
-        if (!sc.ckpt.reserve(lane_floats * lanes * sizeof(float)) ||
-            !cuda_ok(cudaEventRecord(sc.start, s), "fit lanes")) {
-            return LFB_E_CUDA;
-        }
+        if (!cuda_ok(cudaEventRecord(sc.start, s), "fit lanes")) return LFB_E_CUDA;
         int rc = 0;
         for (uint32_t k = 0; k < lanes && !rc; ++k) {
             if (!cuda_ok(cudaStreamWaitEvent(sc.lane[k], sc.start, 0), "fit lanes")) rc = LFB_E_CUDA;

@@ -35,7 +35,6 @@ namespace lfb {
 
 namespace {
 
-constexpr uint32_t kMaxBlock = 256;      // threads of a cell's block, at most
 constexpr uint32_t kCellClauses = 4096;  // arena room per cell, on average
 
 /// Float -> unsigned key with the same order.
@@ -177,57 +176,152 @@ k_pd_boxes(uint32_t n, uint32_t per_cell, uint32_t n_cells, const uint32_t* __re
     }
 }
 
-/// The derivative interpreter (k_derivs) over each cell's own tape: one
-/// block a cell, clauses read two ahead, one float4 (value, partials) per
-/// register and thread.
-__global__ void __launch_bounds__(kMaxBlock)
+/// A clause as the interpreter below reads it: one 16-byte word in shared
+/// memory, constant and free-variable operands already fetched.
+/// x: opcode | PD_* << 8 | result register << 16; y: operand registers a |
+/// b << 16; z, w: the values of immediate operands.
+enum : uint32_t {
+    PD_A_IMM = 1, PD_B_IMM = 2,     // the operand is z / w
+    PD_A_LAST = 4, PD_B_LAST = 8,   // ... is the clause before's result
+    PD_UNARY = 16,
+};
+constexpr uint32_t kPdOps = 64;     // clauses a warp decodes at a time
+
+__device__ __forceinline__ uint4 pd_decode(uint2 raw, uint32_t prev_out, const float* __restrict__ cp)
+{
+    const uint32_t o = raw.x & 0xff, kinds = (raw.x >> 8) & 0xf;
+    const uint32_t a = raw.y & 0xffff, b = raw.y >> 16;
+    uint32_t f = 0;
+    float ia = 0.0f, ib = 0.0f;
+    if ((kinds & 3) != OPND_REG) {
+        f |= PD_A_IMM;
+        ia = __ldg(cp + a);
+    } else if (a == prev_out) {
+        f |= PD_A_LAST;
+    }
+    if (!dev_is_binary(static_cast<uint8_t>(o))) {
+        f |= PD_UNARY;
+    } else if ((kinds >> 2) != OPND_REG) {
+        f |= PD_B_IMM;
+        ib = __ldg(cp + b);
+    } else if (b == prev_out) {
+        f |= PD_B_LAST;
+    }
+    return make_uint4(o | f << 8 | (raw.x & 0xffff0000u), raw.y, __float_as_uint(ia), __float_as_uint(ib));
+}
+
+/// dv_deriv with the square root inline, in dv_deriv_all's operations.
+__device__ __forceinline__ D4 pd_deriv(uint8_t o, const D4& a, const D4& b)
+{
+    if (o != op::SQRT) return dv_deriv(o, a, b, false);
+    const float v = __fsqrt_rn(a.v), den = __fmul_rn(2.0f, v);
+    const bool none = a.v < 0;
+    return {v, none || a.dx == 0 ? 0.0f : __fdiv_rn(a.dx, den),
+            none || a.dy == 0 ? 0.0f : __fdiv_rn(a.dy, den),
+            none || a.dz == 0 ? 0.0f : __fdiv_rn(a.dz, den)};
+}
+
+/// Sort keys of the cells: longest tape first.
+__global__ void k_pd_lengths(const TapeRef* __restrict__ tapes, uint32_t n_cells, uint32_t* keys,
+                             uint32_t* cells)
+{
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n_cells) return;
+    keys[c] = ~tapes[c].len;
+    cells[c] = c;
+}
+
+/// The derivative interpreter over each cell's own tape: one warp for 32 of
+/// its points, one float4 (value, partials) per register and lane.  Tapes'
+/// lengths differ by orders of magnitude, so the warps are blocks of their
+/// own, those of the longest tapes first (with a block a cell, in the
+/// curve's order, the SMs were busy for half of the kernel: 1.45 ms, of
+/// which the instructions need 0.46).  The warp first decodes kPdOps clauses
+/// at a time, a clause a lane, with their constants (the raw words fetched a
+/// chunk ahead), and a result read by the next clause stays in hardware
+/// registers.
+__global__ void __launch_bounds__(32)
 k_pd_derivs(DevTape bt, const TapeRef* __restrict__ tapes, const RegClause* __restrict__ arena,
-            uint32_t n, uint32_t per_cell, const uint32_t* __restrict__ idx,
+            const uint32_t* __restrict__ order, uint32_t n, uint32_t per_cell, const uint32_t* __restrict__ idx,
             const float* __restrict__ X, const float* __restrict__ Y, const float* __restrict__ Z,
             float* __restrict__ ov, float* __restrict__ odx, float* __restrict__ ody,
             float* __restrict__ odz)
 {
     extern __shared__ __align__(16) float4 regs[];
-    float4* R = regs + threadIdx.x;
-    const uint32_t B = blockDim.x;
-    const TapeRef t = tapes[blockIdx.x];
+    __shared__ uint4 ops[kPdOps];
+    constexpr uint32_t B = 32;
+    const uint32_t lane = threadIdx.x;
+    float4* R = regs + lane;
+    const uint32_t cell = order[blockIdx.x / (per_cell / 32)];
+    const uint32_t k = cell * per_cell + blockIdx.x % (per_cell / 32) * 32 + lane;
+    const uint32_t end = min(n, (cell + 1) * per_cell);
+    if (k - lane >= end) return;
+    const TapeRef t = tapes[cell];
     const uint2* cl = reinterpret_cast<const uint2*>(arena + t.off);
     const float* cp = bt.cpool;
-    auto fetch = [&](uint32_t kind, uint32_t r) -> D4 {
-        if (kind == OPND_REG) {
-            const float4 v = R[r * B];
-            return {v.x, v.y, v.z, v.w};
+    const uint2 none = make_uint2(0, 0);
+    auto raw_of = [&](uint32_t c) { return c < t.len ? __ldg(cl + c) : none; };
+    const uint32_t i = idx[min(k, end - 1)];
+    R[0] = make_float4(X[i], 1.0f, 0.0f, 0.0f);
+    R[B] = make_float4(Y[i], 0.0f, 1.0f, 0.0f);
+    R[2 * B] = make_float4(Z[i], 0.0f, 0.0f, 1.0f);
+    D4 last{0.0f, 0.0f, 0.0f, 0.0f};
+    uint2 raw0 = raw_of(lane), raw1 = raw_of(lane + 32);
+    uint32_t before = 0xffffffffu;   // result register of the chunk before's last clause
+    for (uint32_t c0 = 0; c0 < t.len; c0 += kPdOps) {
+        const uint32_t up0 = __shfl_up_sync(0xffffffffu, raw0.x >> 16, 1);
+        const uint32_t mid = __shfl_sync(0xffffffffu, raw0.x >> 16, 31);
+        const uint32_t up1 = __shfl_up_sync(0xffffffffu, raw1.x >> 16, 1);
+        __syncwarp();
+        ops[lane] = pd_decode(raw0, lane ? up0 : before, cp);
+        ops[lane + 32] = pd_decode(raw1, lane ? up1 : mid, cp);
+        before = __shfl_sync(0xffffffffu, raw1.x >> 16, 31);
+        raw0 = raw_of(c0 + kPdOps + lane);
+        raw1 = raw_of(c0 + kPdOps + lane + 32);
+        __syncwarp();
+        const uint32_t m = min(kPdOps, t.len - c0);
+        uint4 next = ops[0];
+#pragma unroll 1
+        for (uint32_t c = 0; c < m; ++c) {
+            const uint4 w = next;
+            next = ops[min(c + 1, kPdOps - 1)];
+            const uint32_t f = w.x >> 8;
+            D4 a, b;
+            if (f & PD_A_LAST) {
+                a = last;
+            } else if (f & PD_A_IMM) {
+                a = {__uint_as_float(w.z), 0.0f, 0.0f, 0.0f};
+            } else {
+                const float4 v = R[(w.y & 0xffff) * B];
+                a = {v.x, v.y, v.z, v.w};
+            }
+            if (f & PD_UNARY) {
+                b = a;
+            } else if (f & PD_B_LAST) {
+                b = last;
+            } else if (f & PD_B_IMM) {
+                b = {__uint_as_float(w.w), 0.0f, 0.0f, 0.0f};
+            } else {
+                const float4 v = R[(w.y >> 16) * B];
+                b = {v.x, v.y, v.z, v.w};
+            }
+            last = pd_deriv(static_cast<uint8_t>(w.x), a, b);
+            R[(w.x >> 16) * B] = make_float4(last.v, last.dx, last.dy, last.dz);
         }
-        return {__ldg(cp + r), 0.0f, 0.0f, 0.0f};
-    };
-    const uint32_t end = min(n, (blockIdx.x + 1) * per_cell);
-    for (uint32_t k0 = blockIdx.x * per_cell; k0 < end; k0 += B) {
-        const uint32_t k = k0 + threadIdx.x;
-        const uint32_t i = idx[min(k, end - 1)];
-        R[0] = make_float4(X[i], 1.0f, 0.0f, 0.0f);
-        R[B] = make_float4(Y[i], 0.0f, 1.0f, 0.0f);
-        R[2 * B] = make_float4(Z[i], 0.0f, 0.0f, 1.0f);
-        const uint2 none = make_uint2(0, 0);
-        uint2 c0 = t.len > 0 ? __ldg(cl) : none, c1 = t.len > 1 ? __ldg(cl + 1) : none;
-        for (uint32_t c = 0; c < t.len; ++c) {
-            const uint2 raw = c0;
-            c0 = c1;
-            if (c + 2 < t.len) c1 = __ldg(cl + c + 2);
-            const uint8_t o = raw.x & 0xff;
-            const uint32_t kinds = (raw.x >> 8) & 0xff;
-            const D4 a = fetch(kinds & 3, raw.y & 0xffff);
-            D4 b = a;
-            if (dev_is_binary(o)) b = fetch((kinds >> 2) & 3, raw.y >> 16);
-            const D4 d = dv_deriv(o, a, b, false);
-            R[(raw.x >> 16) * B] = make_float4(d.v, d.dx, d.dy, d.dz);
+    }
+    if (k < end) {
+        const uint32_t root = t.root & 0xffff;
+        D4 d;
+        if (t.root >> 16 == OPND_REG) {
+            const float4 v = R[root * B];
+            d = {v.x, v.y, v.z, v.w};
+        } else {
+            d = {__ldg(cp + root), 0.0f, 0.0f, 0.0f};
         }
-        if (k < end) {
-            const D4 d = fetch(t.root >> 16, t.root & 0xffff);
-            ov[i] = d.v;
-            if (odx) odx[i] = d.dx;
-            if (ody) ody[i] = d.dy;
-            if (odz) odz[i] = d.dz;
-        }
+        ov[i] = d.v;
+        if (odx) odx[i] = d.dx;
+        if (ody) ody[i] = d.dy;
+        if (odz) odz[i] = d.dz;
     }
 }
 
@@ -284,11 +378,7 @@ bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const
     const uint32_t per_cell =
         std::min<uint32_t>(1024, std::max<uint32_t>(32, (m / (4 * sms) + 31) / 32 * 32));
     const uint32_t n_cells = (m + per_cell - 1) / per_cell;
-    // A thread a point while the register files of two blocks fit an SM.
-    uint32_t block = std::min(kMaxBlock, per_cell);
-    while (block > 32 && bt.n_regs * block * sizeof(float4) > 100 * 1024) block /= 2;
-    block = block / 32 * 32;
-    const size_t file = static_cast<size_t>(bt.n_regs) * block * sizeof(float4);
+    const size_t file = static_cast<size_t>(bt.n_regs) * 32 * sizeof(float4);
     if (!raise_smem_limit(reinterpret_cast<const void*>(k_pd_derivs), file)) {
         clear_error();
         return false;
@@ -299,7 +389,7 @@ bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const
     size_t sort_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<uint32_t*>(nullptr),
                                     static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
-                                    static_cast<uint32_t*>(nullptr), static_cast<int>(m), 0, 30, s);
+                                    static_cast<uint32_t*>(nullptr), static_cast<int>(m), 0, 32, s);
     // One block of scratch in stream order (the pool keeps it, as the
     // mesher's).
     keep_pool_memory(uint64_t(32) << 30);
@@ -311,7 +401,7 @@ bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const
     };
     const size_t o_head = part(256), o_keys = part(4 * n), o_keys2 = part(4 * n),
                  o_idx = part(4 * n), o_idx2 = part(4 * n), o_boxes = part(24 * n_cells),
-                 o_tapes = part(sizeof(TapeRef) * n_cells), o_sort = part(sort_bytes),
+                 o_tapes = part(sizeof(TapeRef) * n_cells), o_order = part(4 * n_cells), o_sort = part(sort_bytes),
                  o_arena = part(8 * arena_cap),
                  o_wide = part(wide_scratch_bytes(bt.n, std::max<uint32_t>(slots, 1)));
     unsigned char* p = nullptr;
@@ -326,6 +416,7 @@ bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const
     uint32_t* keys2 = reinterpret_cast<uint32_t*>(p + o_keys2);
     uint32_t* idx = reinterpret_cast<uint32_t*>(p + o_idx);
     uint32_t* idx2 = reinterpret_cast<uint32_t*>(p + o_idx2);
+    uint32_t* order = reinterpret_cast<uint32_t*>(p + o_order);
     RegClause* arena = reinterpret_cast<RegClause*>(p + o_arena);
     bool ok = cudaMemsetAsync(box, 0xff, 64, s) == cudaSuccess &&
               cudaMemsetAsync(arena_top, 0, 64, s) == cudaSuccess &&
@@ -353,10 +444,16 @@ bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const
     W.n_boxes = n_cells;
     W.box_tape = reinterpret_cast<TapeRef*>(p + o_tapes);
     ok = ok && launch_interval_boxes(W, slots, s) == cudaSuccess;
+    // the keys' buffers again, for the cells' order (n_cells <= n)
     if (ok) {
-        k_pd_derivs<<<n_cells, block, file, s>>>(bt, W.box_tape, arena, m, per_cell, idx2, x, y, z,
-                                                  v, dx, dy, dz);
-        note_launches(5);
+        k_pd_lengths<<<(n_cells + 255) / 256, 256, 0, s>>>(W.box_tape, n_cells, keys, idx);
+        ok = cub::DeviceRadixSort::SortPairs(p + o_sort, sort_bytes, keys, keys2, idx, order,
+                                             static_cast<int>(n_cells), 0, 32, s) == cudaSuccess;
+    }
+    if (ok) {
+        k_pd_derivs<<<n_cells * (per_cell / 32), 32, file, s>>>(bt, W.box_tape, arena, order, m,
+                                                                per_cell, idx2, x, y, z, v, dx, dy, dz);
+        note_launches(6);
     }
     cudaFreeAsync(p, s);
     if (cudaGetLastError() != cudaSuccess) ok = false;
