@@ -793,7 +793,7 @@ std::string bseg_source(const RegTape& t, const JitSeg& sg, uint32_t k,
 
 /// Checkpointed reverse mode, backward kernel (arguments as the backward
 /// kernel's, plus the checkpoints and the constant pool).
-std::string ckpt_backward_source(const RegTape& t)
+std::string ckpt_backward_source(const RegTape& t, bool three)
 {
     const auto segs = jit_segments(t, nullptr);
     std::string body;
@@ -829,16 +829,13 @@ std::string ckpt_backward_source(const RegTape& t)
          "    const unsigned k = lfb_vidx[base + lane];\n"
          "    if (k != 0xffffu && v[0] != 0.0f) atomicAdd(Gv + k, v[0]);\n}\n";
     s += body;
-    // Blocks of 256 threads on an SM: three (80 registers a thread) for
-    // tapes of three or more segments, four (64) for shorter ones.  1,017
-    // clauses, 10^6 points: loss and gradient 838 us with four, 771 with
-    // three, 899 with two; six 377-clause shapes of 65,536 points 166 us with
-    // four, 168 with three.
+    // Blocks of 256 threads on an SM: four (64 registers a thread), or three
+    // (80; ckpt_three).
     // (One 1024-thread block with a barrier before each segment, so that
     // an SM's warps share a segment's instruction fetches, was measured
     // slower: the barriers cost more than the fetch stalls they saved.)
     s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(kCkptBwdBlock) +
-         (segs.size() >= 3 ? ", 3)\n" : ", 4)\n") +
+         (three ? ", 3)\n" : ", 4)\n") +
          "lfb_tape_ckpt_bwd(const float* __restrict__ C, const float* __restrict__ seed,\n"
          "                  float* __restrict__ gx, float* __restrict__ gy,\n"
          "                  float* __restrict__ gz, float* __restrict__ gvars, unsigned m,\n"
@@ -907,8 +904,7 @@ bool build(GpuTape& g, int k, const std::string& src, const char* name)
     return true;
 }
 
-/// The kernel of slot k (0 values, 1 derivatives, 2 reverse-mode
-/// partials, 3 reverse-mode backward pass), compiled on first use.
+/// The kernel of slot k (GpuTape::jit), compiled on first use.
 void* kernel(GpuTape& g, int k, const std::vector<uint32_t>* slots = nullptr)
 {
     std::lock_guard<std::mutex> lock(g.mu);
@@ -926,7 +922,10 @@ void* kernel(GpuTape& g, int k, const std::vector<uint32_t>* slots = nullptr)
                                "lfb_tape_values");
                     break;
                 case 5: ok = build(g, 5, ckpt_forward_source(g.reg), "lfb_tape_ckpt_fwd"); break;
-                case 6: ok = build(g, 6, ckpt_backward_source(g.reg), "lfb_tape_ckpt_bwd"); break;
+                case 6:
+                case 7:
+                    ok = build(g, k, ckpt_backward_source(g.reg, k == 7), "lfb_tape_ckpt_bwd");
+                    break;
                 case 1: ok = build(g, 1, derivs_source(g.reg), "lfb_tape_derivs"); break;
                 case 2: ok = build(g, 2, partials_source(g.reg, *slots), "lfb_tape_partials"); break;
                 case 3: ok = build(g, 3, backward_source(g.reg, *slots), "lfb_tape_backward"); break;
@@ -1034,9 +1033,38 @@ bool jit_backward(GpuTape& g, const uint32_t* slots, uint32_t m, const float* P,
     return launch_1d(fn, m, args, smem, s);
 }
 
-uint32_t jit_ckpt_prepare(GpuTape& g)
+namespace {
+
+/// Whether the backward kernel should run three blocks an SM (80 registers a
+/// thread) instead of four (64).  A wave of three is shorter, 0.69 of the
+/// time at 1,017 clauses, but holds three quarters of the points, so that
+/// the number of waves decides; 0.76 leaves a margin.  1,017 clauses, loss
+/// and gradient with four and three: 10^6 points (7 and 9 waves) 831 and 756
+/// us, 220,000 (2 and 2) 252 and 215, 120,000 (1 and 2) 127 and 149, 800,000
+/// (6 and 8) 651 and 682.  Tapes of one or two segments gain nothing (six
+/// 377-clause shapes of 65,536 points 166 and 168 us).
+bool ckpt_three(const GpuTape& g, uint64_t points)
 {
-    if (!kernel(g, 5) || !kernel(g, 6)) return 0;
+    const uint64_t block = static_cast<uint64_t>(device_sm_count()) * kCkptBwdBlock;
+    const uint64_t w3 = (points + 3 * block - 1) / (3 * block);
+    const uint64_t w4 = (points + 4 * block - 1) / (4 * block);
+    return g.reg.clauses.size() > 2 * kJitSegClauses && 19 * w3 < 25 * w4;
+}
+
+}  // namespace
+
+uint32_t jit_ckpt_prepare(GpuTape& g, uint64_t points)
+{
+    if (!kernel(g, 5)) return 0;
+    // One form is compiled, that of the tape's first call; the one for four
+    // blocks also when a later call has fewer waves with it.
+    bool four, three;
+    {
+        std::lock_guard<std::mutex> lock(g.mu);
+        four = g.jit[6].state == 1;
+    }
+    three = !four && points && ckpt_three(g, points) && kernel(g, 7);
+    if (!three && !kernel(g, 6)) return 0;
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.ckpt_floats) {
         uint32_t total = 0;
@@ -1064,7 +1092,13 @@ bool jit_ckpt_backward(GpuTape& g, uint32_t m, const float* C, const float* seed
     uint32_t n_vars = g.reg.n_vars;
     const unsigned smem = gvars ? n_vars * 4 : 0;
     if (smem > 48 * 1024) return false;
-    void* fn = kernel(g, 6);
+    // the form for this many points, if there are both
+    int k = 6;
+    {
+        std::lock_guard<std::mutex> lock(g.mu);
+        if (g.jit[7].state == 1 && (g.jit[6].state != 1 || ckpt_three(g, m))) k = 7;
+    }
+    void* fn = kernel(g, k);
     if (!fn) return false;
     if (m == 0) return true;
     const float* cp = g.d_cpool;

@@ -65,8 +65,9 @@ struct GpuTape {
         void* module = nullptr;
         void* function = nullptr;
     };
-    // [5] / [6] checkpointed reverse mode, forward / backward
-    JitKernel jit[7];
+    // [5] / [6] checkpointed reverse mode, forward / backward; [7] the
+    // backward pass for three blocks an SM
+    JitKernel jit[8];
     uint32_t ckpt_floats = 0;   // checkpoint slots per point (0: not prepared)
 
     // The CUDA device that was current when the tape was made: its arrays

@@ -1,6 +1,7 @@
 """The branches that work sizes choose: a slice's levels on the list kernels
-or a thread a cell, a height map's rounds over z slabs, and the lanes of a
-fit step; each against the oracle or the same work done one by one."""
+or a thread a cell, a height map's rounds over z slabs, the lanes of a fit
+step, and the reverse mode's two backward kernels; each against the oracle
+or the same work done one by one."""
 import numpy as np
 import pytest
 import torch
@@ -22,7 +23,7 @@ X, Y, Z = Shape.X, Shape.Y, Shape.Z
 @pytest.mark.parametrize("cells", [2, 100, 1500, 6000])
 def test_slice_levels(gpu, cells):
     shape = workloads.spheres_union(64, seed=1)
-    lo, hi, feature = (-1.5, -1.4), (1.3, 1.5), 3.0 / cells
+    lo, hi, feature = (-1.5, -1.5), (1.5, 1.5), 3.0 / cells
     got = render_slice(Tape(shape), lo, hi, 0.05, feature, 1e-8)
     want = oracle_ffi.render_contours(OracleTape(shape), lo, hi, 0.05, feature, 1e-8)[0]
     assert len(got) == len(want)
@@ -30,16 +31,20 @@ def test_slice_levels(gpu, cells):
 
 
 def test_slice_of_many_registers(gpu):
-    # more registers than the list kernels take: a thread a cell throughout
+    # more registers than the list kernels take: a thread a cell throughout.
+    # Every part is read twice, the second time in the same order.
     parts = [(X() * (1.0 + 0.001 * i) + Y() * 0.01 * i).square() + Y().square() - 0.5
-             for i in range(1100)]
-    while len(parts) > 1:
-        half = len(parts) // 2
-        parts = [parts[i].min(parts[i + half]) for i in range(half)] + parts[2 * half:]
-    tape = Tape(parts[0])
+             for i in range(450)]
+    least, most = parts[0], parts[0]
+    for p in parts[1:]:
+        least = least.min(p)
+    for p in parts[1:]:
+        most = most.max(p)
+    shape = least.max(most - 1.0)
+    tape = Tape(shape)
     assert tape.n_regs > 400
     got = render_slice(tape, (-1.5, -1.5), (1.5, 1.5), 0.0, 0.1, 1e-8)
-    want = oracle_ffi.render_contours(OracleTape(parts[0]), (-1.5, -1.5), (1.5, 1.5), 0.0, 0.1, 1e-8)[0]
+    want = oracle_ffi.render_contours(OracleTape(shape), (-1.5, -1.5), (1.5, 1.5), 0.0, 0.1, 1e-8)[0]
     assert same_contours(got, want)
 
 
@@ -81,3 +86,29 @@ def test_fit_side_by_side(gpu, count):
         # component
         g, want = together.m[a:b].cpu().numpy(), alone.m[:b - a].cpu().numpy()
         np.testing.assert_allclose(g, want, rtol=0, atol=1552 * 2.0 ** -24 * 64 * np.abs(want).max())
+
+
+# A tape of more than two segments of 192 clauses, at numbers of points whose
+# first call compiles the backward kernel for three blocks an SM (50,000 and
+# 300,007), or for four (120,001), and then both.
+@pytest.mark.parametrize("sizes", [(50000, 120001, 300007), (120001, 50000)])
+def test_gradient_kernels(gpu, sizes):
+    shape, vals, _ = workloads.fit_csg_vars(32, seed=77)
+    tape, few = Tape(shape, vals), 1000
+    assert tape.n_clauses > 384
+
+    def gradient(t, p):
+        g = [np.zeros(len(p[0]), np.float32) for _ in range(3)]
+        gvars = np.zeros(t.n_vars, np.float32)
+        t.grad(*p, gx=g[0], gy=g[1], gz=g[2], gvars=gvars)
+        return g
+
+    for n in sizes:
+        pts = [np.asarray(a, np.float32) for a in workloads.uniform_points(n, seed=3)]
+        got = gradient(tape, pts)
+        # the points' own gradients are the same numbers from the kernel that
+        # a tape of its own compiles for a few points
+        for at in (0, n - few):
+            want = gradient(Tape(shape, vals), [a[at:at + few] for a in pts])
+            for a, b in zip(got, want):
+                assert np.array_equal(a[at:at + few], b, equal_nan=True)
