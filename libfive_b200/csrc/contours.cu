@@ -864,7 +864,10 @@ bool upload_tables2()
     if (dev < 64 && ((ready >> dev) & 1)) return true;
     DcTables2 t;
     build_dc_tables2(t);
-    if (!cuda_ok(cudaMemcpyToSymbol(c_tab2, &t, sizeof(t)), "contour tables")) return false;
+    if (!cuda_ok(cudaMemcpyToSymbol(c_tab2, &t, sizeof(t)), "contour tables") ||
+        !cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "contour tables")) {
+        return false;
+    }
     if (dev < 64) ready |= 1ull << dev;
     return true;
 }

@@ -2718,7 +2718,10 @@ bool upload_tables()
     if (ready) return true;
     static DcTables t;
     build_dc_tables(t);
-    if (!cuda_ok(cudaMemcpyToSymbol(c_tab, &t, sizeof(t)), "dc tables")) return false;
+    if (!cuda_ok(cudaMemcpyToSymbol(c_tab, &t, sizeof(t)), "dc tables") ||
+        !cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "dc tables")) {
+        return false;
+    }
     ready = true;
     return true;
 }

@@ -384,8 +384,7 @@ bool ensure_pslots(GpuTape& g)
         return false;
     }
     if (!cuda_ok(cudaMalloc(&g.d_pslot, ps.size() * sizeof(uint32_t)), "partial slots") ||
-        !cuda_ok(cudaMemcpy(g.d_pslot, ps.data(), ps.size() * sizeof(uint32_t),
-                            cudaMemcpyHostToDevice), "partial slots")) {
+        !upload(g.d_pslot, ps.data(), ps.size() * sizeof(uint32_t), "partial slots")) {
         return false;
     }
     g.h_pslot = std::move(ps);

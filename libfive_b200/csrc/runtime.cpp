@@ -51,6 +51,14 @@ bool cuda_ok(cudaError_t e, const char* what)
     return false;
 }
 
+bool upload(void* dst, const void* src, size_t bytes, const char* what)
+{
+    // cudaMemcpy from pageable memory returns when the bytes are staged, and
+    // only the legacy stream's work waits for their arrival.
+    return cuda_ok(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what) &&
+           cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), what);
+}
+
 bool require_device()
 {
     static const int state = [] {   // 0 none, 1 ok
@@ -121,8 +129,7 @@ bool GpuTape::ensure_wide()
     const size_t bytes = std::max<size_t>(w.size(), 1) * sizeof(WideEntry);
     if (!cuda_ok(cudaMalloc(&d_wide, bytes), "level-ordered tape alloc")) return false;
     if (!w.empty() &&
-        !cuda_ok(cudaMemcpy(d_wide, w.data(), w.size() * sizeof(WideEntry),
-                            cudaMemcpyHostToDevice), "level-ordered tape upload")) {
+        !upload(d_wide, w.data(), w.size() * sizeof(WideEntry), "level-ordered tape upload")) {
         return false;
     }
     wide_ready = true;
@@ -147,10 +154,7 @@ DevTape GpuTape::dev() const
 bool GpuTape::upload_cpool()
 {
     if (reg.cpool.empty()) return true;
-    return cuda_ok(cudaMemcpy(d_cpool, reg.cpool.data(),
-                              reg.cpool.size() * sizeof(float),
-                              cudaMemcpyHostToDevice),
-                   "upload constants");
+    return upload(d_cpool, reg.cpool.data(), reg.cpool.size() * sizeof(float), "upload constants");
 }
 
 bool GpuTape::pull_vars()
@@ -212,10 +216,8 @@ std::shared_ptr<GpuTape> make_tape(const Tree& t)
         return nullptr;
     }
     if (!g->reg.clauses.empty() &&
-        !cuda_ok(cudaMemcpy(g->d_clauses, g->reg.clauses.data(),
-                            g->reg.clauses.size() * sizeof(RegClause),
-                            cudaMemcpyHostToDevice),
-                 "tape upload")) {
+        !upload(g->d_clauses, g->reg.clauses.data(), g->reg.clauses.size() * sizeof(RegClause),
+                "tape upload")) {
         return nullptr;
     }
     if (!g->upload_cpool()) {

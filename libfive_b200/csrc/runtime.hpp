@@ -26,6 +26,9 @@ bool require_device();
 
 /// Converts a CUDA status into an error record; returns true on success.
 bool cuda_ok(cudaError_t e, const char* what);
+/// Copies host data to the device; when it returns, work on any stream finds
+/// it there.
+bool upload(void* dst, const void* src, size_t bytes, const char* what);
 
 /// memcpy between host blocks over a few threads: one thread moves (and
 /// first touches) a large mesh's arrays several times slower than the GPU
