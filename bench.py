@@ -408,8 +408,8 @@ def run_ours(args, world, rank, local):
                      "triangles": stats.triangles, "vertices": stats.vertices,
                      "leaf_records": stats.leaves_ambiguous},
             "roofline": {
-                "kernel": "leaf stage: k_leaf_groups (corners, edge search; 82 % of the "
-                          "stage) + k_leaf_qef + k_edge_rank + k_leaf_vertices",
+                "kernel": "leaf stage: k_leaf_decode + k_leaf_groups (corners, edge search) + "
+                          "k_leaf_qef + k_edge_rank + k_leaf_vertices",
                 "bound": "fp32",
                 "achieved": achieved, "peak": peak, "unit": "G lane-ops/s",
                 "frac": achieved / peak,
@@ -422,8 +422,7 @@ def run_ours(args, world, rank, local):
                 "traffic_source": ("ncu capture of the leaf stage's four kernels on this "
                                    "workload, dram__bytes_read.sum + dram__bytes_write.sum "
                                    "(profiles/k_leaf_groups_csg2000_depth10_dram.md), taken "
-                                   "before the edge-slot cleanup of k_leaf_groups: an upper "
-                                   "bound for the current kernels"
+                                   "before the leaf stage ran in fused steps"
                                    if traffic is not None else None),
             },
             "stages_ms": {"interval": stats.ms_interval, "leaf": stats.ms_leaf,
