@@ -1046,6 +1046,7 @@ struct __align__(16) LeafWarpShared {
 struct LeafWarpScratch {
     FeatureScratch fs;
     EdgeSlot e[54];
+    uint32_t check_status;   // of the feature searches at listed zeros
 };
 
 /// A crossing lattice edge's QEF, handed from the leaf kernel to the rank
@@ -1063,9 +1064,10 @@ struct GroupEdges {
     uint32_t base;          // 0xffffffff: the records did not fit
     uint32_t zbase;         // its zero-valued samples in LeafArgs::zeros
     uint8_t n_edges;
-    uint8_t n_zeros;
+    uint8_t n_zeros;        // or kZerosRedo
     int8_t slot_of[54];
 };
+constexpr uint8_t kZerosRedo = 0xff;   // the group is on the redo list
 
 /// The interpreters' register file (one float4 per register and lane): in
 /// the block's dynamic shared memory at byte offset `soff` (S = true: the
@@ -1720,9 +1722,9 @@ k_leaf_groups(const __grid_constant__ LeafArgs A, uint32_t n_groups)
             }
             if (n_zeros > kLeafZeros || zbase > A.zero_cap || n_zeros > A.zero_cap - zbase) {
                 if (lane == 0) A.redo[atomicAdd(A.n_redo, 1u)] = g;
-                n_zeros = 0;
+                n_zeros = kZerosRedo;
             }
-            for (uint32_t k = lane; k < 3 * n_zeros; k += 32) {
+            for (uint32_t k = lane; n_zeros != kZerosRedo && k < 3 * n_zeros; k += 32) {
                 A.zeros[size_t{3} * zbase + k] = S->zpt[k / 3][k % 3];
             }
         }
@@ -1767,6 +1769,11 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
     const FeatCtx fc{A.featws + (static_cast<size_t>(blockIdx.x) * wpb + warp) *
                                     A.bt.n_regs * kRegBlock,
                      &W->fs, A.status};
+    // A listed zero may lie where the careful search never comes (after one
+    // that is not inside), so a feature search that overflows there sends the
+    // group back instead of failing the mesh.
+    const FeatCtx check_fc{fc.regs, fc.tmp, &W->check_status};
+    if (!REDO && lane == 0) W->check_status = 0;
     uint64_t my_devals = 0;
     const Octree& o = A.o;
     const int Ld = o.levels;
@@ -1781,7 +1788,7 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
         const GroupEdges& ge = A.group_edges[single ? 0 : g];
         const uint32_t gbase = ge.base;
         const int E = ge.n_edges;
-        if (gbase == 0xffffffffu || E == 0) continue;
+        if (gbase == 0xffffffffu || E == 0 || (!REDO && ge.n_zeros == kZerosRedo)) continue;
         const TapeRef tr = single ? root_tape_ref(A.bt) : o.lv[Ld].group_tape[g];
         const RegClause* cl = A.arena + tr.off;
         const DevTape tb = with_tape(A.bt, tr);
@@ -1819,13 +1826,20 @@ k_leaf_qef(LeafArgs A, uint32_t n_groups)
             const float gr[3] = {d.dx, d.dy, d.dz};
             outside |= check && !amb && !(sqrtf(fdot(gr, gr)) > 0);
             uint32_t pending = __ballot_sync(0xffffffffu, check && amb);
+            const bool searched = pending != 0;
             while (pending) {
                 const int src = __ffs(pending) - 1;
                 pending &= pending - 1;
                 const float fx = __shfl_sync(0xffffffffu, q[0], src);
                 const float fy = __shfl_sync(0xffffffffu, q[1], src);
                 const float fz = __shfl_sync(0xffffffffu, q[2], src);
-                outside |= !dev_is_inside(fc, tb, cl, tr.len, fx, fy, fz, lane);
+                outside |= !dev_is_inside(check_fc, tb, cl, tr.len, fx, fy, fz, lane);
+            }
+            if (searched) {
+                __syncwarp();
+                uint32_t overflowed = 0;
+                if (lane == 0) overflowed = atomicExch(&W->check_status, 0u);
+                outside |= __shfl_sync(0xffffffffu, overflowed, 0) != 0;
             }
             if (active) {
                 EdgeSlot& es = W->e[p >> 1];
