@@ -94,11 +94,12 @@ __device__ __forceinline__ WideConsts wide_consts(const uint4& e, const float* _
 
 /// Interval of list entry k, stored in slot 3 + k, and the entry's state for
 /// the cell's children; returns whether a min/max got decided
-/// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167); nan_safe:
-/// not between operands that may be NaN.
+/// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167); enclosing:
+/// intervals enclose what the point interpreters compute, and nothing is
+/// decided between operands that may be NaN.
 __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c, uint32_t k,
                                              float2* S, uint8_t* SN, uint8_t* pst,
-                                             bool nan_safe = false)
+                                             bool enclosing = false)
 {
     const uint8_t o = e.x & 0xff;
     const uint32_t kinds = (e.x >> 8) & 0xf;
@@ -114,11 +115,12 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
         const Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
         const Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
         r = iv_eval(o, a, b);
+        if (enclosing) r = iv_enclose(o, a, b, r);
         if (o == op::MIN || o == op::MAX) {
             uint8_t keep = 0;   // 0 both, 1 a, 2 b
             if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;
             else if (b.lo > a.hi) keep = (o == op::MAX) ? 2 : 1;
-            if (keep && !(nan_safe && (a.nan || b.nan))) {
+            if (keep && !(enclosing && (a.nan || b.nan))) {
                 ps = keep == 1 ? WIDE_A : WIDE_B;
                 decided = true;
             }

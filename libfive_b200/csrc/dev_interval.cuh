@@ -490,6 +490,19 @@ __device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
     }
 }
 
+/// r = iv_eval(o, a, b) made an enclosure of every value that the point
+/// interpreters compute for operands in a and b.  The rules above are the
+/// reference's, which a mesh needs to be its mesh; where they leave values
+/// out, a min / max decided by them can drop the operand that a point takes:
+///  * a reciprocal over an interval that ends at zero is a half line, but
+///    the zero at its end has either sign (1 / +0 = inf in [-1, 0]).
+__device__ __forceinline__ Iv iv_enclose(uint8_t o, const Iv& a, const Iv& b, Iv r)
+{
+    (void)b;
+    if (o == op::RECIP && a.lo <= 0.0f && a.hi >= 0.0f) r = {-LF_INF, LF_INF, a.nan};
+    return r;
+}
+
 /// Interval::state(): AMBIGUOUS when the value may be NaN.
 enum : uint8_t { ST_EMPTY = 0, ST_FILLED = 1, ST_AMBIGUOUS = 2, ST_UNKNOWN = 3 };
 __device__ __forceinline__ uint8_t iv_state(const Iv& a)

@@ -1,0 +1,48 @@
+"""Derivatives of long tapes pruned per cell of points, where an operation's
+interval ends at a value at which the operation jumps or overflows: the whole
+tape's values and partials, bit for bit, taken from calls too small for the
+pruned path."""
+import numpy as np
+import pytest
+
+from libfive_b200 import workloads as wl
+from libfive_b200.shape import Shape, Tape, X, Y, Z
+
+pytestmark = pytest.mark.gpu
+
+
+def long_tape(s):
+    """s over a union of spheres that makes the tape too long to be compiled
+    and has values between -2 and 4 in the region of the points; the sum
+    reads both everywhere."""
+    tape = Tape(wl.spheres_union(400, seed=9) + s)
+    assert tape.n_clauses > 4096
+    return tape
+
+
+def same_as_whole_tape(tape, p):
+    got = tape.derivs(*p)
+    parts = [tape.derivs(*[np.ascontiguousarray(c[i:i + 255]) for c in p]) for i in range(0, len(p[0]), 255)]
+    want = [np.concatenate([q[k] for q in parts]) for k in range(4)]
+    return all(np.array_equal(a.view(np.uint32)[~np.isnan(b)], b.view(np.uint32)[~np.isnan(b)]) and
+               np.array_equal(np.isnan(a), np.isnan(b)) for a, b in zip(got, want))
+
+
+def points_ending_at_zero(sign, zero, n=4096):
+    """Half of the points at x = zero, the others on one side of it, so that
+    many cells' boxes end there."""
+    rng = np.random.default_rng(5)
+    x = (sign * rng.uniform(0.0, 0.9, n)).astype(np.float32)
+    x[rng.random(n) < 0.5] = zero
+    y, z = (rng.uniform(-1.0, 1.0, n).astype(np.float32) for _ in range(2))
+    return x, y, z
+
+
+# min(1 / x, -1) below x = 0 and max(1 / x, 1) above it: the whole tape takes
+# the constant at a zero of the other side's sign.
+@pytest.mark.parametrize("zero", [0.0, -0.0])
+@pytest.mark.parametrize("sign", [-1.0, 1.0])
+def test_reciprocal_up_to_zero(gpu, sign, zero):
+    r = Shape.new("recip", X())
+    tape = long_tape(r.min(-1.0).max(-50.0) if sign < 0 else r.max(1.0).min(50.0))
+    assert same_as_whole_tape(tape, points_ending_at_zero(sign, np.float32(zero)))
