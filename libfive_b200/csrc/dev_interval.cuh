@@ -495,10 +495,12 @@ __device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
 /// reference's, which a mesh needs to be its mesh; where they leave values
 /// out, a min / max decided by them can drop the operand that a point takes:
 ///  * a reciprocal over an interval that ends at zero is a half line, but
-///    the zero at its end has either sign (1 / +0 = inf in [-1, 0]).
+///    the zero at its end has either sign (1 / +0 = inf in [-1, 0]);
+///  * a difference of two intervals that both reach +inf may be NaN (where
+///    both reach -inf the rule says so).
 __device__ __forceinline__ Iv iv_enclose(uint8_t o, const Iv& a, const Iv& b, Iv r)
 {
-    (void)b;
+    if (o == op::SUB && a.hi == LF_INF && b.hi == LF_INF) r.nan = true;
     if (o == op::RECIP && a.lo <= 0.0f && a.hi >= 0.0f) r = {-LF_INF, LF_INF, a.nan};
     return r;
 }

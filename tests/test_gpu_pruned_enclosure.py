@@ -46,3 +46,17 @@ def test_reciprocal_up_to_zero(gpu, sign, zero):
     r = Shape.new("recip", X())
     tape = long_tape(r.min(-1.0).max(-50.0) if sign < 0 else r.max(1.0).min(50.0))
     assert same_as_whole_tape(tape, points_ending_at_zero(sign, np.float32(zero)))
+
+
+# inf - inf is NaN at the points of a corner, where both terms overflow; its
+# absolute value is never below zero, and so decides against -1 unless the
+# interval says that it may be NaN.
+def test_difference_of_infinities(gpu):
+    d = ((X() * 100.0).exp() - (Y() * 100.0).exp()).abs()
+    tape = long_tape(d.min(-1.0) + (-d).max(1.0))
+    x, y, z = (np.random.default_rng(a).uniform(0.8, 1.0, 4096).astype(np.float32) for a in range(3))
+    assert same_as_whole_tape(tape, (x, y, z))
+    # infinite coordinates under a linear difference
+    tape = long_tape((X() * 0.8 - Y() * 0.6).square().min(-1.0))
+    x[::7], y[::7] = np.inf, np.inf
+    assert same_as_whole_tape(tape, (x, y, z))
