@@ -112,8 +112,12 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
     } else if (st == WIDE_B) {
         r = wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN);
     } else {
-        const Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
-        const Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
+        Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
+        Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
+        if (enclosing) {
+            a = iv_not_empty(a);   // a constant or variable that is NaN
+            b = iv_not_empty(b);
+        }
         r = iv_eval(o, a, b);
         if (enclosing) r = iv_enclose(o, a, b, r);
         if (o == op::MIN || o == op::MAX) {
@@ -631,7 +635,7 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
         if (tid < 3) {
             Iv v;
             if (boxes) {
-                v = iv_make(A.boxes[6 * i + 2 * tid], A.boxes[6 * i + 2 * tid + 1]);
+                v = iv_not_empty(iv_make(A.boxes[6 * i + 2 * tid], A.boxes[6 * i + 2 * tid + 1]));
             } else {
                 double blo[3], bhi[3];
                 cell_bounds(o, d, lv.coords[i], blo, bhi);

@@ -490,6 +490,11 @@ __device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
     }
 }
 
+__device__ __forceinline__ Iv iv_not_empty(const Iv& a)
+{
+    return iv_bad(a) ? Iv{-LF_INF, LF_INF, true} : a;
+}
+
 /// r = iv_eval(o, a, b) made an enclosure of every value that the point
 /// interpreters compute for operands in a and b.  The rules above are the
 /// reference's, which a mesh needs to be its mesh; where they leave values
@@ -497,12 +502,15 @@ __device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
 ///  * a reciprocal over an interval that ends at zero is a half line, but
 ///    the zero at its end has either sign (1 / +0 = inf in [-1, 0]);
 ///  * a difference of two intervals that both reach +inf may be NaN (where
-///    both reach -inf the rule says so).
+///    both reach -inf the rule says so);
+///  * the empty interval ([NaN, NaN]), which the rules read as "always NaN":
+///    log(x <= 0) is -inf at zero, and a box with NaN coordinates stands for
+///    points that have none, too.  It becomes the whole line, maybe NaN.
 __device__ __forceinline__ Iv iv_enclose(uint8_t o, const Iv& a, const Iv& b, Iv r)
 {
     if (o == op::SUB && a.hi == LF_INF && b.hi == LF_INF) r.nan = true;
     if (o == op::RECIP && a.lo <= 0.0f && a.hi >= 0.0f) r = {-LF_INF, LF_INF, a.nan};
-    return r;
+    return iv_not_empty(r);
 }
 
 /// Interval::state(): AMBIGUOUS when the value may be NaN.

@@ -60,3 +60,23 @@ def test_difference_of_infinities(gpu):
     tape = long_tape((X() * 0.8 - Y() * 0.6).square().min(-1.0))
     x[::7], y[::7] = np.inf, np.inf
     assert same_as_whole_tape(tape, (x, y, z))
+
+
+# log(x) over [lo, 0] is -inf at the points at zero and NaN at the others: as
+# a second operand of min it is the value at zero, although the other operand
+# is the value elsewhere.
+@pytest.mark.parametrize("zero", [0.0, -0.0])
+def test_logarithm_up_to_zero(gpu, zero):
+    one = Shape.constant(1.0)
+    tape = long_tape(one.min(X().log()).max(0.5))
+    assert same_as_whole_tape(tape, points_ending_at_zero(-1.0, np.float32(zero)))
+
+
+# Cells with a few points that have a NaN coordinate, or a NaN constant.
+def test_nan_among_others(gpu):
+    one = Shape.constant(1.0)
+    x, y, z = (np.random.default_rng(a).uniform(-3.0, 0.0, 4096).astype(np.float32) for a in range(3))
+    x[100], y[200], z[300] = np.nan, np.nan, np.nan
+    assert same_as_whole_tape(long_tape(one.min(X()).max(0.5) + one.min(Y() + Z()).max(-0.5)), (x, y, z))
+    nan = Shape.constant(float("nan"))
+    assert same_as_whole_tape(long_tape(one.min(X() + nan).max(0.5)), (x, y, z))
