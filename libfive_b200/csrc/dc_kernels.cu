@@ -112,14 +112,9 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
     } else if (st == WIDE_B) {
         r = wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN);
     } else {
-        Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
-        Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
-        if (enclosing) {
-            a = iv_not_empty(a);   // a constant or variable that is NaN
-            b = iv_not_empty(b);
-        }
+        const Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
+        const Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
         r = iv_eval(o, a, b);
-        if (enclosing) r = iv_enclose(o, a, b, r);
         if (o == op::MIN || o == op::MAX) {
             uint8_t keep = 0;   // 0 both, 1 a, 2 b
             if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;
@@ -128,6 +123,8 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
                 ps = keep == 1 ? WIDE_A : WIDE_B;
                 decided = true;
             }
+        } else if (enclosing) {
+            r = iv_enclose(o, a, b, r);
         }
     }
     S[3 + k] = make_float2(r.lo, r.hi);

@@ -506,6 +506,8 @@ __device__ __forceinline__ Iv iv_not_empty(const Iv& a)
 ///  * the empty interval ([NaN, NaN]), which the rules read as "always NaN":
 ///    log(x <= 0) is -inf at zero, and a box with NaN coordinates stands for
 ///    points that have none, too.  It becomes the whole line, maybe NaN.
+/// min and max need none of it: of operands that are not empty, or a
+/// constant that is NaN, they enclose what a point takes.
 __device__ __forceinline__ Iv iv_enclose(uint8_t o, const Iv& a, const Iv& b, Iv r)
 {
     if (o == op::SUB && a.hi == LF_INF && b.hi == LF_INF) r.nan = true;

@@ -327,7 +327,8 @@ k_pd_derivs(DevTape bt, const TapeRef* __restrict__ tapes, const RegClause* __re
 
 /// Whether every clause's interval rule encloses what the derivative
 /// interpreter computes: directed-rounding operations, and exp and log,
-/// whose bounds are widened past their error.
+/// whose bounds are widened past their error; all of them as iv_enclose
+/// (dev_interval.cuh) corrects them.
 bool sound_ops(GpuTape& g)
 {
     std::lock_guard<std::mutex> lock(g.mu);

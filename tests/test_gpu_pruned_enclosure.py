@@ -80,3 +80,44 @@ def test_nan_among_others(gpu):
     assert same_as_whole_tape(long_tape(one.min(X()).max(0.5) + one.min(Y() + Z()).max(-0.5)), (x, y, z))
     nan = Shape.constant(float("nan"))
     assert same_as_whole_tape(long_tape(one.min(X() + nan).max(0.5)), (x, y, z))
+
+
+UNARY = ("square", "sqrt", "neg", "abs", "recip", "exp", "log", "const-var")
+BINARY = ("add", "sub", "mul", "div", "min", "max")
+SPECIAL = (0.0, -0.0, 1.0, -1.0, 88.0, 3e38, -3e38, 1e-40, np.inf, -np.inf, np.nan)
+
+
+def random_tree(rng, depth):
+    if depth == 0:
+        if rng.random() < 0.2:
+            return Shape.constant(float(rng.choice(SPECIAL)))
+        # a factor of its own, so that no two subtrees are one
+        return (X, Y, Z)[rng.integers(3)]() * float(rng.uniform(0.5, 2.0))
+    if rng.random() < 0.35:
+        return Shape.new(str(rng.choice(UNARY)), random_tree(rng, depth - 1))
+    op = str(rng.choice(BINARY if rng.random() < 0.5 else BINARY[4:]))
+    return Shape.new(op, random_tree(rng, depth - 1), random_tree(rng, depth - 1))
+
+
+# Every operation that the pruned path takes, over constants and coordinates
+# at its edges: 500 trees, joined twelve at a time and those one by one.
+@pytest.mark.parametrize("seed", [0, 1, 2, 3])
+def test_random_trees(gpu, seed):
+    rng = np.random.default_rng(seed)
+    parts = [random_tree(rng, int(rng.integers(3, 6))) for _ in range(500)]
+    parts = [t.min(0.01 * i) if i % 2 else Shape.constant(-0.01 * i).max(t) for i, t in enumerate(parts)]
+    for width in (12, 50):
+        parts = [parts[i:i + width] for i in range(0, len(parts), width)]
+        for p in parts:
+            while len(p) > 1:
+                p[:2] = [p[0].min(p[1]) if rng.random() < 0.5 else p[0].max(p[1])]
+        parts = [p[0] for p in parts]
+    tape = Tape(parts[0])
+    assert tape.n_clauses > 4096 and tape.n_regs <= 100 and tape.n_choices >= tape.n_clauses // 64
+    p = []
+    for _ in range(3):
+        v = (rng.uniform(-2.0, 2.0, 5000) * (1.0, 1e-3, 100.0, 1e19)[seed]).astype(np.float32)
+        at = rng.random(5000) < 0.15
+        v[at] = rng.choice(np.array(SPECIAL, np.float32), at.sum())
+        p.append(v)
+    assert same_as_whole_tape(tape, p)
