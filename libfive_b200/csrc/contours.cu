@@ -895,6 +895,28 @@ struct ContourBuffers {
         b.ordered = true;   // from the device's memory pool, on the default stream
         return b.reserve(std::max<size_t>(count, 1) * sizeof(T)) ? b.as<T>() : nullptr;
     }
+    /// Elements that the kept buffer holds.
+    template <class T>
+    uint64_t holds(int key)
+    {
+        return bufs[key].bytes / sizeof(T);
+    }
+    /// A larger buffer with the first `keep` elements of the old one.
+    template <class T>
+    T* grow(int key, size_t count, size_t keep)
+    {
+        DevBuf old;
+        DevBuf& b = bufs[key];
+        std::swap(old.ptr, b.ptr);
+        std::swap(old.bytes, b.bytes);
+        old.ordered = true;
+        T* p = get<T>(key, count);
+        if (p && !cuda_ok(cudaMemcpyAsync(p, old.ptr, keep * sizeof(T), cudaMemcpyDeviceToDevice, nullptr),
+                          "contour arena")) {
+            p = nullptr;
+        }
+        return p;   // the old one is freed in stream order
+    }
     void trim()
     {
         size_t total = 0;
@@ -1013,10 +1035,28 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
     const bool lists_ok = bt.n && bt.n_regs <= kMaxTapeRegs && g.ensure_wide();
     if (!lists_ok) clear_error();
 
-    uint64_t arena_cap = std::max<uint64_t>(static_cast<uint64_t>(bt.n) * 64, 1u << 20);
-    uint64_t list_cap = 4ull * bt.n + 1024;
-    uint32_t rec_cap = 1u << 16, task_cap = 1u << 18, seg_cap = 1u << 16;
-    for (int attempt = 0; attempt < 6; ++attempt) {
+    // Capacities: what the kept buffers hold, or a usual slice's needs.  The
+    // arena and the lists grow at the level that overflows them, which is
+    // then run again; records, tasks and segments grow to what was counted,
+    // and the slice is started again.
+    const bool small = debug_hooks().small_capacity.load() != 0;
+    auto capacity = [&](uint64_t least, uint64_t usual, uint64_t kept) {
+        return small ? least : std::max(usual, kept);
+    };
+    uint64_t arena_cap = capacity(bt.n + 16, std::max<uint64_t>(static_cast<uint64_t>(bt.n) * 64, 1u << 20),
+                                  B.holds<RegClause>(CB::ARENA));
+    uint64_t list_cap[2];   // by parity of the depth that reads them
+    for (int k = 0; k < 2; ++k) {
+        list_cap[k] = capacity(16, 4ull * bt.n + 1024, B.holds<WideEntry>(k ? CB::LISTS_B : CB::LISTS_A));
+    }
+    const uint64_t most_entries = small ? 64ull * bt.n : uint64_t(1) << 25;   // of one level's lists
+    constexpr uint64_t kMostCount = uint64_t(1) << 30;   // records, tasks, segments: 32-bit counts
+    uint64_t rec_cap = capacity(64, 1u << 16, B.holds<QLeaf>(CB::RECS));
+    uint64_t task_cap = capacity(64, 1u << 18, std::min(B.holds<QTask>(CB::TASKS_A), B.holds<QTask>(CB::TASKS_B)));
+    uint64_t seg_cap = capacity(64, 1u << 16, B.holds<uint2>(CB::SEGS));
+    auto more = [](uint64_t cap, uint64_t count) { return std::max(2 * cap, count + count / 4); };
+    for (int attempt = 0; attempt < 24; ++attempt) {
+        if (std::max({rec_cap, task_cap, seg_cap}) > kMostCount) break;
         const size_t tr_bytes = static_cast<size_t>(nregs) * T;
         RegClause* arena = B.get<RegClause>(CB::ARENA, arena_cap);
         unsigned long long* ctr = B.get<unsigned long long>(CB::CTR, 8);
@@ -1104,7 +1144,6 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
             W.arena_top = arena_top;
             W.arena_cap = arena_cap;
             W.out_top = ctr + 5;
-            W.out_cap = list_cap;
             W.status = status;
             W.next_cell = reinterpret_cast<uint32_t*>(ctr + 6);
             W.group_shift = 2;
@@ -1117,14 +1156,14 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
             if (!ql[0].coords || !ql[1].coords || !ql[0].group_tape || !ql[1].group_tape ||
                 !ql[0].group_list || !ql[1].group_list ||
                 !B.get<ListRef>(CB::CELL_LIST, kListCells) ||
-                !B.get<WideEntry>(CB::LISTS_A, list_cap) || !B.get<WideEntry>(CB::LISTS_B, list_cap)) {
+                !B.get<WideEntry>(CB::LISTS_A, list_cap[0]) || !B.get<WideEntry>(CB::LISTS_B, list_cap[1])) {
                 return LFB_E_CUDA;
             }
             cudaMemsetAsync(ql[0].coords, 0, sizeof(uint64_t), s);
         }
 
         // quadtree build, level by level
-        bool list_overflow = false, arena_overflow = false;
+        unsigned long long arena_used = bt.n;
         for (int d = 0; d < L; ++d) {
             const uint32_t n = t.lv[d].n;
             if (n == 0) {
@@ -1141,54 +1180,86 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
             if (!out_tape || !flags || !scan || !tmp) return LFB_E_CUDA;
             lists = lists && n < kListCells;
             ListRef* cell_list = nullptr;
-            if (lists) {
-                LevelView& lv = W.o.lv[d];
-                cell_list = B.get<ListRef>(CB::CELL_LIST, n);
-                lv = LevelView{};
-                lv.n_cells = n;
-                lv.coords = ql[d & 1].coords;
-                lv.type = t.lv[d].type;
-                lv.cell_tape = out_tape;
-                lv.cell_list = cell_list;
-                lv.group_tape = ql[d & 1].group_tape;
-                lv.group_list = ql[d & 1].group_list;
-                W.in_lists = d == 0 ? g.d_wide
-                                    : B.get<WideEntry>(d & 1 ? CB::LISTS_B : CB::LISTS_A, list_cap);
-                W.out_lists = B.get<WideEntry>(d & 1 ? CB::LISTS_A : CB::LISTS_B, list_cap);
-                W.write_lists = d + 1 < L;
-                cudaMemsetAsync(ctr + 5, 0, 16, s);
-                if (!cuda_ok(launch_interval_lists(W, d, n, wide_warps, s), "contour intervals")) {
+            uint32_t n_branch = 0;
+            for (int again = 0;; ++again) {
+                if (lists) {
+                    LevelView& lv = W.o.lv[d];
+                    cell_list = B.get<ListRef>(CB::CELL_LIST, n);
+                    lv = LevelView{};
+                    lv.n_cells = n;
+                    lv.coords = ql[d & 1].coords;
+                    lv.type = t.lv[d].type;
+                    lv.cell_tape = out_tape;
+                    lv.cell_list = cell_list;
+                    lv.group_tape = ql[d & 1].group_tape;
+                    lv.group_list = ql[d & 1].group_list;
+                    const int out = (d + 1) & 1;
+                    W.in_lists = d == 0 ? g.d_wide : B.get<WideEntry>(out ? CB::LISTS_A : CB::LISTS_B, 1);
+                    W.out_lists = B.get<WideEntry>(out ? CB::LISTS_B : CB::LISTS_A, list_cap[out]);
+                    if (!W.in_lists || !W.out_lists) return LFB_E_CUDA;
+                    W.out_cap = list_cap[out];
+                    W.write_lists = d + 1 < L;
+                    W.arena = arena;
+                    W.arena_cap = arena_cap;
+                    cudaMemsetAsync(ctr + 5, 0, 16, s);
+                    if (!cuda_ok(launch_interval_lists(W, d, n, wide_warps, s), "contour intervals")) {
+                        return LFB_E_CUDA;
+                    }
+                } else {
+                    QIntervalArgs A{t, d, bt, arena, arena_top, arena_cap, out_tape, rlo, rhi,
+                                    rnan, live, dec, dec_cap, T, status};
+                    k_q_interval<<<std::min<uint32_t>(T / 256, (n + 255) / 256), 256, 0, s>>>(A);
+                }
+                k_q_branch_flags<<<(n + 256) / 256, 256, 0, s>>>(t.lv[d].type, n, flags);
+                note_launches(2);
+                unsigned long long seen[8];   // ctr
+                if (!cuda_ok(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flags, scan, n + 1, s), "scan") ||
+                    !cuda_ok(cudaMemcpyAsync(&n_branch, scan + n, 4, cudaMemcpyDeviceToHost, s), "download") ||
+                    !cuda_ok(cudaMemcpyAsync(seen, ctr, sizeof(seen), cudaMemcpyDeviceToHost, s), "download") ||
+                    !cuda_ok(cudaStreamSynchronize(s), "contour intervals")) {
                     return LFB_E_CUDA;
                 }
-            } else {
-                QIntervalArgs A{t, d, bt, arena, arena_top, arena_cap, out_tape, rlo, rhi,
-                                rnan, live, dec, dec_cap, T, status};
-                k_q_interval<<<std::min<uint32_t>(T / 256, (n + 255) / 256), 256, 0, s>>>(A);
+                const uint32_t st = static_cast<uint32_t>(seen[2]);
+                if (!(st & (ST_LIST_OVERFLOW | ST_ARENA_OVERFLOW))) {
+                    arena_used = seen[0];
+                    break;
+                }
+                // The counters kept counting past the capacity: room for what
+                // this level needs, and again.
+                if (again == 3 || seen[0] >> 32) {
+                    return set_error(LFB_E_CAPACITY, "contours: tape arena overflow");
+                }
+                if (st & ST_LIST_OVERFLOW) {
+                    // Lists that do not get shorter (shapes without a min or
+                    // max to decide) are copied cell by cell: past
+                    // most_entries, 512 MiB, a thread a cell goes on without
+                    // them.  The bound is for memory: lists are the faster
+                    // form at every size measured (200 blended spheres,
+                    // depth 11, lists of up to 12 M entries: 180 ms, given up
+                    // at 3 M 203 ms, at 0.3 M 232 ms).
+                    const int out = (d + 1) & 1;
+                    if (seen[5] > most_entries) lists = false;
+                    else list_cap[out] = seen[5] + seen[5] / 4 + 1024;
+                    cell_list = nullptr;
+                }
+                if (st & ST_ARENA_OVERFLOW) {
+                    arena_cap = seen[0] + seen[0] / 4 + (1u << 20);
+                    arena = B.grow<RegClause>(CB::ARENA, arena_cap, arena_used);
+                    if (!arena) return LFB_E_CUDA;
+                }
+                const uint32_t others = st & ~(ST_LIST_OVERFLOW | ST_ARENA_OVERFLOW);
+                cudaMemcpyAsync(arena_top, &arena_used, sizeof(arena_used), cudaMemcpyHostToDevice, s);
+                cudaMemcpyAsync(status, &others, sizeof(others), cudaMemcpyHostToDevice, s);
             }
-            k_q_branch_flags<<<(n + 256) / 256, 256, 0, s>>>(t.lv[d].type, n, flags);
-            note_launches(2);
-            uint32_t n_branch = 0, st = 0;
-            if (!cuda_ok(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flags, scan, n + 1, s), "scan") ||
-                !cuda_ok(cudaMemcpyAsync(&n_branch, scan + n, 4, cudaMemcpyDeviceToHost, s), "download") ||
-                !cuda_ok(cudaMemcpyAsync(&st, status, 4, cudaMemcpyDeviceToHost, s), "download") ||
-                !cuda_ok(cudaStreamSynchronize(s), "contour intervals")) {
-                return LFB_E_CUDA;
-            }
-            list_overflow = (st & ST_LIST_OVERFLOW) != 0;
-            arena_overflow = (st & ST_ARENA_OVERFLOW) != 0;
-            if (list_overflow || arena_overflow) break;
             if (!alloc_level(d + 1, 4 * n_branch)) return LFB_E_CUDA;
             k_q_children<<<(n + 255) / 256, 256, 0, s>>>(t, d, scan, out_tape, cell_list, ql[(d + 1) & 1]);
             note_launches(1);
             if (!cuda_ok(cudaGetLastError(), "contour intervals")) return LFB_E_CUDA;
         }
-        if (list_overflow) list_cap *= 4;
-        if (arena_overflow) arena_cap *= 4;
-        if (list_overflow || arena_overflow) continue;
 
         // leaves at the finest depth
         if (t.lv[L].n) {
-            QLeafArgs A{t, bt, arena, lregs, nregs, featws, fs, recs_d, rec_top, rec_cap, status};
+            QLeafArgs A{t, bt, arena, lregs, nregs, featws, fs, recs_d, rec_top, static_cast<uint32_t>(rec_cap), status};
             const uint32_t blocks = std::min<uint32_t>(leaf_warps / kLeafWarps,
                                                        (t.lv[L].n + kLeafWarps - 1) / kLeafWarps);
             k_q_leaf<<<std::max<uint32_t>(blocks, 1), 32 * kLeafWarps, 0, s>>>(A);
@@ -1196,7 +1267,7 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         }
         // collapse, bottom-up
         for (int d = L - 1; d >= 0; --d) {
-            QCollapseArgs C{t, d, bt, arena, recs_d, rec_top, rec_cap, max_err,
+            QCollapseArgs C{t, d, bt, arena, recs_d, rec_top, static_cast<uint32_t>(rec_cap), max_err,
                             cregs, T, status};
             k_q_collapse<<<T / 256, 256, 0, s>>>(C);
             note_launches(1);
@@ -1204,15 +1275,19 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
         uint32_t st = 0;
         cudaMemcpyAsync(&st, status, 4, cudaMemcpyDeviceToHost, s);
         if (!cuda_ok(cudaStreamSynchronize(s), "contour leaves")) return LFB_E_CUDA;
-        if (st & ST_ARENA_OVERFLOW) { arena_cap *= 4; continue; }
-        if (st & ST_RECORD_OVERFLOW) { rec_cap *= 4; continue; }
+        if (st & ST_RECORD_OVERFLOW) {
+            uint32_t count = 0;
+            if (!cuda_ok(cudaMemcpy(&count, rec_top, 4, cudaMemcpyDeviceToHost), "contour leaves")) return LFB_E_CUDA;
+            rec_cap = more(rec_cap, count);
+            continue;
+        }
         if (st & (ST_FEATURE_OVERFLOW | ST_REGS)) {
             return set_error(LFB_E_CAPACITY, "contours: feature list or decision capacity exceeded");
         }
 
         // dual walk
-        QDualArgs D{t, recs_d, tasks_a, n_tasks, task_cap,
-                    segs_d, n_segs, seg_cap, status};
+        QDualArgs D{t, recs_d, tasks_a, n_tasks, static_cast<uint32_t>(task_cap),
+                    segs_d, n_segs, static_cast<uint32_t>(seg_cap), status};
         for (int d = 0; d < L; ++d) {
             if (t.lv[d].n) k_q_dual_init<<<(t.lv[d].n + 255) / 256, 256, 0, s>>>(D, d);
             note_launches(1);
@@ -1236,8 +1311,10 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
             std::swap(qa, qb);
         }
         if (overflow) {
-            task_cap *= 4;
-            seg_cap *= 4;
+            uint32_t count = 0;
+            if (!cuda_ok(cudaMemcpy(&count, n_segs, 4, cudaMemcpyDeviceToHost), "contour walk")) return LFB_E_CUDA;
+            if (n_in > task_cap) task_cap = more(task_cap, n_in);
+            if (count > seg_cap) seg_cap = more(seg_cap, count);
             continue;
         }
         uint32_t ns = 0, nr = 0;
