@@ -1008,7 +1008,7 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
     cudaStream_t s = 0;
 
     ContourBuffers& B = contour_buffers();
-    std::lock_guard<std::mutex> lock(B.mu);
+    std::unique_lock<std::mutex> lock(B.mu);
     int dev = 0;
     if (!cuda_ok(cudaGetDevice(&dev), "device")) return LFB_E_CUDA;
     if (B.device != dev) {
@@ -1021,8 +1021,15 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
     }
     struct Trim {
         ContourBuffers& b;
-        ~Trim() { b.trim(); }
-    } trim{B};
+        std::unique_lock<std::mutex>& lock;
+        void done()
+        {
+            if (!lock.owns_lock()) return;
+            b.trim();
+            lock.unlock();
+        }
+        ~Trim() { done(); }
+    } buffers_in_use{B, lock};
     using CB = ContourBuffers;
 
     // The list kernels take the first levels, while there are fewer cells
@@ -1329,6 +1336,9 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
                                        cudaMemcpyDeviceToHost), "download"))) {
             return LFB_E_CUDA;
         }
+        // The rest is host work on this call's own arrays: the next call may
+        // have the buffers.
+        buffers_in_use.done();
         std::vector<std::pair<uint32_t, uint32_t>> sp(ns);
         for (uint32_t k = 0; k < ns; ++k) sp[k] = {segs[k].x, segs[k].y};
         std::vector<std::vector<uint32_t>> welded;
