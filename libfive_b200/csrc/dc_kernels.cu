@@ -1026,7 +1026,8 @@ constexpr uint32_t kLeafSteps = 56;   // steps of a tape in shared memory at a t
 constexpr uint32_t kLeafChunk = 4;    // groups taken at a time, with 16 or more a warp
 
 /// Per-warp state of the corner and edge-search kernel, in shared memory
-/// (24 warps an SM beside register files of kLeafSmemRegsMany registers).
+/// (24 warps an SM beside register files of kLeafSmemRegsMany registers, 16
+/// beside kLeafSmemRegs).
 struct __align__(16) LeafWarpShared {
     union {
         ValOp vops[kLeafSteps];    // the tape's steps (short tapes: once a group)
@@ -1200,14 +1201,11 @@ static __device__ __noinline__ D4 leaf_deriv(const float* __restrict__ cpool, ui
     return {__ldg(cpool + root), 0.0f, 0.0f, 0.0f};
 }
 
-// Registers of the shared-memory register file per warp.  k_leaf_groups:
-// 8 when the groups fill the GPU (9.5 KB a warp, 24 warps an SM; 99 % of the
-// leaf tapes of CSG models use at most 8 registers, the others run from
-// global memory), 16 when all its warps fit beside each other anyway (at
-// most kLeafFewGroups groups); k_leaf_qef: 16.
+// Registers of the shared-memory register file per warp, 16 or 8 in
+// k_leaf_groups (16 warps an SM or 24) and 16 in k_leaf_qef; longer tapes'
+// groups run from global memory, clause by clause.
 constexpr uint32_t kLeafSmemRegs = 16;
 constexpr uint32_t kLeafSmemRegsMany = 8;
-constexpr uint32_t kLeafFewGroups = 148 * 16;
 constexpr int kLeafWarps = 8, kLeafBlocks = 3;   // warps per block, blocks per SM
 static_assert(kLeafSmemRegs <= kValMaxRegs, "register offsets of a step are 16 bits");
 
@@ -2492,6 +2490,9 @@ struct MeshCounters {
     uint32_t n_groups;       // branch cells of the level
     uint32_t nregs;          // largest register count of their tapes
     uint32_t pad;
+    // clauses of their tapes (the last level's): of up to 8 registers, of
+    // 9 to 16 and of more
+    unsigned long long clauses[3];
     // leaf stage
     uint32_t next_group, next_group2;
     uint32_t zero_top, n_redo;
@@ -2513,15 +2514,28 @@ __global__ void k_init_root(Octree o, MeshCounters* c, uint32_t n_clauses)
 
 /// Flags of the branch cells (flags[n] = 0), how many there are and the
 /// largest register count of their tapes (which sizes the group-mode
-/// interval kernel's shared memory for the next depth).
+/// interval kernel's shared memory for the next depth); of the last level
+/// also their clauses by register count (which size the leaf kernel's).
 __global__ void k_branch_flags(const uint8_t* type, const TapeRef* cell_tape, uint32_t n,
-                               uint32_t* flags, MeshCounters* c)
+                               uint32_t* flags, MeshCounters* c, bool last)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool branch = i < n && type[i] == CELL_BRANCH;
     if (i <= n) flags[i] = branch ? 1u : 0u;
     const uint32_t count = __popc(__ballot_sync(0xffffffffu, branch));
-    const uint32_t most = __reduce_max_sync(0xffffffffu, branch ? cell_tape[i].nregs : 0u);
+    const uint32_t nregs = branch ? cell_tape[i].nregs : 0u;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, nregs);
+    if (last) {
+        __shared__ unsigned long long sums[3];
+        if (threadIdx.x < 3) sums[threadIdx.x] = 0;
+        __syncthreads();
+        if (branch) {
+            atomicAdd(sums + (nregs <= kLeafSmemRegsMany ? 0 : nregs <= kLeafSmemRegs ? 1 : 2),
+                      static_cast<unsigned long long>(cell_tape[i].len));
+        }
+        __syncthreads();
+        if (threadIdx.x < 3 && sums[threadIdx.x]) atomicAdd(c->clauses + threadIdx.x, sums[threadIdx.x]);
+    }
     if ((threadIdx.x & 31) == 0 && count) {
         atomicAdd(&c->n_groups, count);
         atomicMax(&c->nregs, most);
@@ -3321,7 +3335,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             // The level's counts go back while the branch cells are scanned:
             // one wait per level.
             k_branch_flags<<<lv.n_cells / 256 + 1, 256, 0, s>>>(lv.type, lv.cell_tape, lv.n_cells,
-                                                                flags, counters);
+                                                                flags, counters, d + 1 == L);
             ++n_launch;
             if (!fetch_counters("interval kernel") || !exclusive_scan(ws, flags, scan, lv.n_cells + 1, s) ||
                 !cuda_ok(cudaStreamSynchronize(s), "interval kernel")) {
@@ -3439,9 +3453,19 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         }
         // Shared memory: per warp its state and a register file of smem_regs
         // float4s a lane; groups whose tape needs more registers use global
-        // memory instead.
+        // memory instead.  Sixteen registers where all warps then fit beside
+        // each other anyway (16 an SM), and where the tapes of 9 to 16 gain
+        // more than the others lose with fewer warps an SM.  Leaf stage with
+        // 8 and 16 registers, ms: all clauses in tapes of 9 to 16 (16 and 64
+        // smooth blends) 9.8 and 7.9, 81 and 67; of up to 8 (CSG of 1,000)
+        // 5.7 and 6.1; of more than 16 (blends with min) 119 and 141.  CSG of
+        // 2,000 with 67 % of the clauses in tapes of 9 to 16 24.4 and 23.5, of
+        // 4,000 with 21 % 78 and 81: hence the weights.
+        const unsigned long long* clauses = seen.clauses;
+        const bool few = n_leaf_groups <= sms * 16;
         const uint32_t group_regs = std::min<uint32_t>(
-            bt.n_regs, n_leaf_groups <= kLeafFewGroups ? kLeafSmemRegs : kLeafSmemRegsMany);
+            bt.n_regs, few || 2 * clauses[1] > clauses[0] + 3 * clauses[2] ? kLeafSmemRegs
+                                                                           : kLeafSmemRegsMany);
         const uint32_t qef_regs = std::min<uint32_t>(bt.n_regs, kLeafSmemRegs);
         const size_t group_bytes = (sizeof(LeafWarpShared) + size_t{512} * group_regs) * wpb;
         const size_t qef_bytes = (sizeof(LeafOp) * kLeafOps + size_t{512} * qef_regs) * wpb;
@@ -3540,10 +3564,10 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         ++n_launch;
         if (L > 0) {
             // the groups a check sent back (usually none)
-            const uint32_t few = std::min(grid, sms);
+            const uint32_t few_blocks = std::min(grid, sms);
             A.smem_regs = group_regs;
             A.chunk = 1;
-            redo_kernel<<<few, 32 * wpb, group_bytes, s>>>(A, n_leaf_groups);
+            redo_kernel<<<few_blocks, 32 * wpb, group_bytes, s>>>(A, n_leaf_groups);
             A.smem_regs = qef_regs;
             k_leaf_qef<true><<<std::min(qef_grid, sms), 32 * wpb, qef_bytes, s>>>(A, n_leaf_groups);
             n_launch += 2;
