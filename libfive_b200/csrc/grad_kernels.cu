@@ -464,7 +464,7 @@ int grad_device(GpuTape& g, uint64_t n, const float* x, const float* y, const fl
     // Checkpointed reverse mode when the tape compiles: per point it stores
     // only the registers each tape segment reads from earlier segments, and
     // the backward kernel recomputes the segment from them (jit.cpp).
-    if (const uint32_t ckf = jit_ckpt_prepare(g, n)) {
+    if (const uint32_t ckf = jit_ckpt_prepare(g)) {
         const uint64_t per_point = 4ull * ckf;
         const uint64_t cchunk = std::max<uint64_t>(kBlock, std::min<uint64_t>(
             (4ull << 30) / per_point / kBlock * kBlock, uint64_t(1) << 22));
@@ -606,7 +606,7 @@ bool grad_prepare(GpuTape& g)
 {
     // the checkpointed kernels, which grad_device takes when they compile;
     // else the stored-partials kernels (m = 0: compile, no launch)
-    if (jit_ckpt_prepare(g, 0)) return true;
+    if (jit_ckpt_prepare(g)) return true;
     if (!ensure_pslots(g)) return false;
     const uint32_t* hs = g.h_pslot.data();
     jit_partials(g, hs, 0, nullptr, nullptr, nullptr, nullptr, nullptr, 0);
@@ -672,7 +672,7 @@ int eval_loss_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const
     auto& st = grad_staging();
     if (!st.out.reserve(sizeof(double))) return LFB_E_CUDA;
     double* sum = st.out.as<double>();
-    if (const uint32_t ckf = jit_ckpt_prepare(g, n)) {
+    if (const uint32_t ckf = jit_ckpt_prepare(g)) {
         // one forward pass gives f and the checkpoints; the backward pass
         // takes seed 2 f_i / n
         const uint64_t per_point = 4ull * ckf;
@@ -721,7 +721,7 @@ int eval_loss_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const
 
 uint64_t grad_scratch_floats(GpuTape& g, uint64_t n)
 {
-    const uint32_t ckf = tape_has_const_var(g) ? 0 : jit_ckpt_prepare(g, 0);
+    const uint32_t ckf = tape_has_const_var(g) ? 0 : jit_ckpt_prepare(g);
     // one launch pair: no more points than grad_device takes at once
     return ckf && n <= (uint64_t(1) << 22) ? n * ckf : 0;
 }

@@ -8,8 +8,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -884,14 +887,10 @@ bool iv_supported(uint8_t o)
     return op::arity(o) >= 1;
 }
 
-/// Compiles `src` and loads its kernel `name` into slot k; false when
-/// anything is unavailable or fails.
-bool build(GpuTape& g, int k, const std::string& src, const char* name)
+/// Loads kernel `name` of a compiled module into slot k.
+bool load(GpuTape& g, int k, const std::vector<char>& cubin, const char* name)
 {
     const Api& A = api();
-    if (!A.ok || src.empty()) return false;
-    std::vector<char> cubin;
-    if (!jit_compile(src, &cubin, nullptr)) return false;
     CUmodule mod = nullptr;
     CUfunction fn = nullptr;
     if (A.load(&mod, cubin.data()) != CUDA_SUCCESS) return false;
@@ -904,27 +903,77 @@ bool build(GpuTape& g, int k, const std::string& src, const char* name)
     return true;
 }
 
+/// Compiles `src` and loads its kernel `name` into slot k; false when
+/// anything is unavailable or fails.
+bool build(GpuTape& g, int k, const std::string& src, const char* name)
+{
+    std::vector<char> cubin;
+    return api().ok && !src.empty() && jit_compile(src, &cubin, nullptr) && load(g, k, cubin, name);
+}
+
+/// Whether a tape's backward kernel also has the form for three blocks an SM
+/// (ckpt_three).
+bool has_ckpt_three(const GpuTape& g) { return g.reg.clauses.size() > 2 * kJitSegClauses; }
+
+/// Compiles the checkpointed reverse mode's kernels that the tape has, each
+/// on a thread of its own, so that a later call never waits for a compiler
+/// whatever its number of points.  With g.mu held.
+void build_ckpt(GpuTape& g)
+{
+    struct Job {
+        int k;
+        std::string src;
+        std::vector<char> cubin;
+        bool ok;
+    };
+    std::vector<Job> jobs;
+    const bool fits = api().ok && g.reg.clauses.size() <= kJitMaxSegmentedClauses;
+    for (int k = 5; k <= (has_ckpt_three(g) ? 7 : 6); ++k) {
+        if (g.jit[k].state) continue;
+        g.jit[k].state = -1;
+        if (fits) jobs.push_back({k, k == 5 ? ckpt_forward_source(g.reg) : ckpt_backward_source(g.reg, k == 7), {}, false});
+    }
+    auto compile = [](Job& j) {
+        try {
+            j.ok = !j.src.empty() && jit_compile(j.src, &j.cubin, nullptr);
+        } catch (const std::exception&) {   // not out of a thread
+        }
+    };
+    std::thread other[3];
+    for (size_t i = 1; i < jobs.size(); ++i) {
+        try {
+            other[i] = std::thread(compile, std::ref(jobs[i]));
+        } catch (const std::system_error&) {
+            compile(jobs[i]);   // no thread to be had: here
+        }
+    }
+    if (!jobs.empty()) compile(jobs[0]);
+    for (auto& t : other) {
+        if (t.joinable()) t.join();
+    }
+    for (Job& j : jobs) {
+        if (j.ok && load(g, j.k, j.cubin, j.k == 5 ? "lfb_tape_ckpt_fwd" : "lfb_tape_ckpt_bwd")) g.jit[j.k].state = 1;
+    }
+}
+
 /// The kernel of slot k (GpuTape::jit), compiled on first use.
 void* kernel(GpuTape& g, int k, const std::vector<uint32_t>* slots = nullptr)
 {
     std::lock_guard<std::mutex> lock(g.mu);
     GpuTape::JitKernel& j = g.jit[k];
-    if (j.state == 0) {
+    if (j.state == 0 && k >= 5) {
+        build_ckpt(g);
+    } else if (j.state == 0) {
         const size_t n = g.reg.clauses.size();
         bool ok = api().ok && n <= (k == 4 ? kJitMaxIntervalClauses
-                                    : (k == 0 || k >= 5) ? kJitMaxSegmentedClauses
-                                                         : kJitMaxClauses);
+                                    : k == 0 ? kJitMaxSegmentedClauses
+                                             : kJitMaxClauses);
         if (ok) {
             switch (k) {
                 case 0:
                     ok = build(g, 0, n <= kJitMaxClauses ? values_source(g.reg)
                                                          : values_source_segmented(g.reg),
                                "lfb_tape_values");
-                    break;
-                case 5: ok = build(g, 5, ckpt_forward_source(g.reg), "lfb_tape_ckpt_fwd"); break;
-                case 6:
-                case 7:
-                    ok = build(g, k, ckpt_backward_source(g.reg, k == 7), "lfb_tape_ckpt_bwd");
                     break;
                 case 1: ok = build(g, 1, derivs_source(g.reg), "lfb_tape_derivs"); break;
                 case 2: ok = build(g, 2, partials_source(g.reg, *slots), "lfb_tape_partials"); break;
@@ -1048,23 +1097,14 @@ bool ckpt_three(const GpuTape& g, uint64_t points)
     const uint64_t block = static_cast<uint64_t>(device_sm_count()) * kCkptBwdBlock;
     const uint64_t w3 = (points + 3 * block - 1) / (3 * block);
     const uint64_t w4 = (points + 4 * block - 1) / (4 * block);
-    return g.reg.clauses.size() > 2 * kJitSegClauses && 19 * w3 < 25 * w4;
+    return has_ckpt_three(g) && 19 * w3 < 25 * w4;
 }
 
 }  // namespace
 
-uint32_t jit_ckpt_prepare(GpuTape& g, uint64_t points)
+uint32_t jit_ckpt_prepare(GpuTape& g)
 {
-    if (!kernel(g, 5)) return 0;
-    // One form is compiled, that of the tape's first call; the one for four
-    // blocks also when a later call has fewer waves with it.
-    bool four, three;
-    {
-        std::lock_guard<std::mutex> lock(g.mu);
-        four = g.jit[6].state == 1;
-    }
-    three = !four && points && ckpt_three(g, points) && kernel(g, 7);
-    if (!three && !kernel(g, 6)) return 0;
+    if (!kernel(g, 5) || !kernel(g, 6)) return 0;
     std::lock_guard<std::mutex> lock(g.mu);
     if (!g.ckpt_floats) {
         uint32_t total = 0;
@@ -1092,13 +1132,8 @@ bool jit_ckpt_backward(GpuTape& g, uint32_t m, const float* C, const float* seed
     uint32_t n_vars = g.reg.n_vars;
     const unsigned smem = gvars ? n_vars * 4 : 0;
     if (smem > 48 * 1024) return false;
-    // the form for this many points, if there are both
-    int k = 6;
-    {
-        std::lock_guard<std::mutex> lock(g.mu);
-        if (g.jit[7].state == 1 && (g.jit[6].state != 1 || ckpt_three(g, m))) k = 7;
-    }
-    void* fn = kernel(g, k);
+    void* fn = ckpt_three(g, m) ? kernel(g, 7) : nullptr;
+    if (!fn) fn = kernel(g, 6);
     if (!fn) return false;
     if (m == 0) return true;
     const float* cp = g.d_cpool;

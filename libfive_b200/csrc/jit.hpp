@@ -78,10 +78,11 @@ bool jit_compile(const std::string& src, std::vector<char>* cubin, std::string* 
 /// segments (C[slot * m + i], jit_ckpt_prepare's count of slots); the
 /// backward kernel recomputes each segment from them and sweeps its
 /// adjoints back, with the products and sums of the partials / backward
-/// kernels.  jit_ckpt_prepare compiles both (the backward kernel in the form
-/// for `points` points) and returns the slot count, or 0 when the tape has no
-/// compiled form.
-uint32_t jit_ckpt_prepare(GpuTape& g, uint64_t points);
+/// kernels.  jit_ckpt_prepare compiles both (the backward kernel of longer
+/// tapes in two forms, of which each call takes the one for its number of
+/// points) and returns the slot count, or 0 when the tape has no compiled
+/// form.
+uint32_t jit_ckpt_prepare(GpuTape& g);
 bool jit_ckpt_forward(GpuTape& g, uint32_t m, const float* x, const float* y, const float* z,
                       float* C, float* f, cudaStream_t s);
 /// The seed of point i is seed[i] (1 when seed is null) times seed_scale.
