@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "eval_api.hpp"
+#include "jit.hpp"
 #include "libfive_b200.h"
 
 namespace lfb {
@@ -251,10 +252,20 @@ int fit_adam_step(GpuTape* const* tapes, uint32_t n_shapes, const uint64_t* poff
     // shapes run on up to eight lanes that branch off the caller's stream
     // and join it again: 6 shapes of 65,536 points 219 -> 167 us a step.
     // Shapes without the checkpointed form, or whose checkpoints do not fit
-    // the lanes' scratch, run one after another.
+    // the lanes' scratch, run one after another; so do two or three shapes
+    // that leave nothing idle (jit_ckpt_fills_gpu), whose kernels only take the
+    // instruction cache from each other: two of 2,844 clauses at 57,344
+    // points 473 us side by side and 332 one after another, two of 1,844 at
+    // 81,920 289 and 258.  Six such shapes gain by fewer tails (1,035 and
+    // 1,161), two of 947 clauses are the same (148 and 156).
     uint64_t lane_floats = 0;
     const uint32_t lanes = std::min(kFitLanes, n_shapes);
     bool side_by_side = n_shapes > 1;
+    if (n_shapes <= 3) {
+        uint32_t full = 0;
+        for (uint32_t j = 0; j < n_shapes; ++j) full += jit_ckpt_fills_gpu(*tapes[j], poff[j + 1] - poff[j]);
+        side_by_side = side_by_side && full < n_shapes;
+    }
     for (uint32_t j = 0; j < n_shapes && side_by_side; ++j) {
         const uint64_t c = grad_scratch_floats(*tapes[j], poff[j + 1] - poff[j]);
         lane_floats = std::max(lane_floats, c);

@@ -1102,6 +1102,12 @@ bool ckpt_three(const GpuTape& g, uint64_t points)
 
 }  // namespace
 
+bool jit_ckpt_fills_gpu(const GpuTape& g, uint64_t points)
+{
+    const uint64_t wave = 3ull * static_cast<uint64_t>(device_sm_count()) * kCkptBwdBlock;
+    return g.reg.clauses.size() > 8 * kJitSegClauses && 2 * points > wave && points <= wave;
+}
+
 uint32_t jit_ckpt_prepare(GpuTape& g)
 {
     if (!kernel(g, 5) || !kernel(g, 6)) return 0;

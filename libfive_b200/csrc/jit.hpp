@@ -83,6 +83,10 @@ bool jit_compile(const std::string& src, std::vector<char>* cubin, std::string* 
 /// points) and returns the slot count, or 0 when the tape has no compiled
 /// form.
 uint32_t jit_ckpt_prepare(GpuTape& g);
+/// Whether `points` points of a long tape keep the GPU busy by themselves: one
+/// wave of the backward kernel that is more than half full, with code that
+/// fills the instruction cache.
+bool jit_ckpt_fills_gpu(const GpuTape& g, uint64_t points);
 bool jit_ckpt_forward(GpuTape& g, uint32_t m, const float* x, const float* y, const float* z,
                       float* C, float* f, cudaStream_t s);
 /// The seed of point i is seed[i] (1 when seed is null) times seed_scale.
