@@ -277,7 +277,19 @@ int fit_adam_step(GpuTape* const* tapes, uint32_t n_shapes, const uint64_t* poff
         clear_error();
         side_by_side = false;
     }
-    if (side_by_side) {
+    // A stream being captured keeps to itself: lanes that joined its capture
+    // would stay in it until its end, and the next fit's with them.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) cudaGetLastError();
+    if (side_by_side && capturing != cudaStreamCaptureStatusNone) {
+        for (uint32_t j = 0; j < n_shapes; ++j) {
+            float* gv = voff[j + 1] > voff[j] ? grad + (voff[j] - v0) : nullptr;
+            if (int rc = eval_grad_with(*tapes[j], poff[j + 1] - poff[j], x + poff[j], y + poff[j],
+                                        z + poff[j], f + (poff[j] - p0), gv, sc.ckpt.as<float>(), s)) {
+                return rc;
+            }
+        }
+    } else if (side_by_side) {
         if (!cuda_ok(cudaEventRecord(sc.start, s), "fit lanes")) return LFB_E_CUDA;
         int rc = 0;
         for (uint32_t k = 0; k < lanes && !rc; ++k) {
