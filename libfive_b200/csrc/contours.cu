@@ -865,7 +865,7 @@ bool upload_tables2()
     DcTables2 t;
     build_dc_tables2(t);
     if (!cuda_ok(cudaMemcpyToSymbol(c_tab2, &t, sizeof(t)), "contour tables") ||
-        !cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "contour tables")) {
+        !uploaded("contour tables")) {
         return false;
     }
     if (dev < 64) ready |= 1ull << dev;

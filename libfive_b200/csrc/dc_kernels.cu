@@ -2750,7 +2750,7 @@ bool upload_tables()
     static DcTables t;
     build_dc_tables(t);
     if (!cuda_ok(cudaMemcpyToSymbol(c_tab, &t, sizeof(t)), "dc tables") ||
-        !cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "dc tables")) {
+        !uploaded("dc tables")) {
         return false;
     }
     ready = true;

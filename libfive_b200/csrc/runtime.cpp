@@ -51,12 +51,22 @@ bool cuda_ok(cudaError_t e, const char* what)
     return false;
 }
 
+bool uploaded(const char* what)
+{
+    // Relaxed, as the copy itself is: a capture on another stream forbids the
+    // wait otherwise (variables may be set while one is open).
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return cuda_ok(e, what);
+}
+
 bool upload(void* dst, const void* src, size_t bytes, const char* what)
 {
     // cudaMemcpy from pageable memory returns when the bytes are staged, and
     // only the legacy stream's work waits for their arrival.
-    return cuda_ok(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what) &&
-           cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), what);
+    return cuda_ok(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what) && uploaded(what);
 }
 
 bool require_device()

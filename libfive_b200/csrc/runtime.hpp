@@ -29,6 +29,8 @@ bool cuda_ok(cudaError_t e, const char* what);
 /// Copies host data to the device; when it returns, work on any stream finds
 /// it there.
 bool upload(void* dst, const void* src, size_t bytes, const char* what);
+/// Waits for the copies from pageable memory made so far.
+bool uploaded(const char* what);
 
 /// memcpy between host blocks over a few threads: one thread moves (and
 /// first touches) a large mesh's arrays several times slower than the GPU
