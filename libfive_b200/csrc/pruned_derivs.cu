@@ -369,6 +369,7 @@ bool pruned_derivs(GpuTape& g, uint64_t n, const float* x, const float* y, const
         cudaGetLastError();
         return false;   // the general path allocates nothing
     }
+    RelaxedCapture relaxed;   // another stream's capture may be open
     if (!g.ensure_wide()) {
         clear_error();
         return false;

@@ -53,13 +53,10 @@ bool cuda_ok(cudaError_t e, const char* what)
 
 bool uploaded(const char* what)
 {
-    // Relaxed, as the copy itself is: a capture on another stream forbids the
-    // wait otherwise (variables may be set while one is open).
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    return cuda_ok(e, what);
+    // Relaxed, as the copy itself is: variables may be set while a capture is
+    // open.
+    RelaxedCapture relaxed;
+    return cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), what);
 }
 
 bool upload(void* dst, const void* src, size_t bytes, const char* what)

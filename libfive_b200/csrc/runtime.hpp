@@ -26,6 +26,18 @@ bool require_device();
 
 /// Converts a CUDA status into an error record; returns true on success.
 bool cuda_ok(cudaError_t e, const char* what);
+/// While one lives, an open capture on another stream does not forbid this
+/// thread's allocations and waits, which take no part in it.
+class RelaxedCapture {
+  public:
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+  private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
 /// Copies host data to the device; when it returns, work on any stream finds
 /// it there.
 bool upload(void* dst, const void* src, size_t bytes, const char* what);
