@@ -181,9 +181,10 @@ int lfb_fit_adam_step(const lfb_tape* tapes, uint32_t n_shapes,
  *  error below which cells collapse (negative disables collapsing).
  *  cancel (NULL: none): BRepSettings::cancel (settings.hpp:73); the mesher
  *  reads it between octree levels, before the leaf and collapse stages and
- *  before the launch of each dual-walk round, and when it is non-zero stops, releases what
- *  the call holds and fails with LFB_E_CANCELLED (the reference returns a
- *  null mesh, worker_pool.inl:82-85, mesh.cpp:61-66). */
+ *  before and after the dual walk (whose rounds are launched together), and
+ *  when it is non-zero stops, releases what the call holds and fails with
+ *  LFB_E_CANCELLED (the reference returns a null mesh,
+ *  worker_pool.inl:82-85, mesh.cpp:61-66). */
 typedef struct lfb_mesh_settings {
     double min_feature;
     double max_err;

@@ -3698,6 +3698,7 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
                 !cuda_ok(cudaStreamSynchronize(s), "dual walk")) {
                 return LFB_E_CUDA;
             }
+            if (cancelled()) return LFB_E_CANCELLED;   // raised during the walk
             if (seen.status & ST_QUEUE_OVERFLOW) {
                 task_cap *= 4;
                 tri_cap *= 4;
