@@ -2672,6 +2672,9 @@ struct Workspace {
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
     MeshCounters* seen = nullptr;   // page-locked: the counters as last read
+    // The mesh is rendered again after the device ran out of memory: it does
+    // without what it can do without.
+    bool lean = false;
     // Leaf edge records per leaf group (grows when a mesh needs more; the
     // mesh is then rendered again).
     uint32_t edges_per_group = 16;
@@ -3463,9 +3466,30 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         // 4,000 with 21 % 78 and 81: hence the weights.
         const unsigned long long* clauses = seen.clauses;
         const bool few = n_leaf_groups <= sms * 16;
-        const uint32_t group_regs = std::min<uint32_t>(
+        uint32_t group_regs = std::min<uint32_t>(
             bt.n_regs, few || 2 * clauses[1] > clauses[0] + 3 * clauses[2] ? kLeafSmemRegs
                                                                            : kLeafSmemRegsMany);
+        // Steps by clause offset, so room for as many as the arena has
+        // clauses: 36 bytes beside each clause's own 8.  Where no tape can be
+        // decoded, or the device has no such room left even for a mesh that is
+        // rendered again by itself, every group runs from global memory,
+        // clause by clause.
+        ValOp* vops = nullptr;
+        uint32_t* n_steps = nullptr;
+        const bool decodable = L == 0 ? bt.n_regs <= group_regs
+                                      : clauses[0] + (group_regs > kLeafSmemRegsMany ? clauses[1] : 0) != 0;
+        if (decodable) {
+            vops = ws.get<ValOp>(K_VOPS, arena_used);
+            n_steps = ws.get<uint32_t>(K_NSTEPS, arena_used);
+        }
+        if (!vops || !n_steps) {
+            if (decodable && !ws.lean) return LFB_E_CUDA;
+            take_device_oom();
+            clear_error();
+            group_regs = 0;
+        } else {
+            cudaMemsetAsync(n_steps, 0, arena_used * sizeof(uint32_t), s);
+        }
         const uint32_t qef_regs = std::min<uint32_t>(bt.n_regs, kLeafSmemRegs);
         const size_t group_bytes = (sizeof(LeafWarpShared) + size_t{512} * group_regs) * wpb;
         const size_t qef_bytes = (sizeof(LeafOp) * kLeafOps + size_t{512} * qef_regs) * wpb;
@@ -3522,11 +3546,6 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
         GroupEdges* gedges = ws.get<GroupEdges>(K_GEDGES, n_leaf_groups);
         uint32_t* rec_group = ws.get<uint32_t>(K_RECGROUP, rec_cap);
         if (!edges || !gedges || !rec_group) return LFB_E_CUDA;
-        // Steps by clause offset, so room for as many as the arena has clauses.
-        ValOp* vops = ws.get<ValOp>(K_VOPS, arena_used);
-        uint32_t* n_steps = ws.get<uint32_t>(K_NSTEPS, arena_used);
-        if (!vops || !n_steps) return LFB_E_CUDA;
-        cudaMemsetAsync(n_steps, 0, arena_used * sizeof(uint32_t), s);
         // Zero-valued samples: room for 32 a group on average (none with the
         // small-capacity hook, so that every such group is searched again).
         const uint32_t zero_cap = small ? 0u : static_cast<uint32_t>(std::min<uint64_t>(
@@ -3552,11 +3571,13 @@ int render_once(Workspace& ws, GpuTape& g, const libfive_region3& R, double min_
             }
             tapes = t;
         }
-        // groups per decoding warp: as few as fill the GPU
-        const uint32_t per_warp = std::min(32u, n_leaf_groups / (sms * 32) + 1);
-        k_leaf_decode<<<(n_leaf_groups + 4 * per_warp - 1) / (4 * per_warp), 128, 0, s>>>(
-            A, tapes, n_leaf_groups, per_warp);
-        ++n_launch;
+        if (group_regs) {
+            // groups per decoding warp: as few as fill the GPU
+            const uint32_t per_warp = std::min(32u, n_leaf_groups / (sms * 32) + 1);
+            k_leaf_decode<<<(n_leaf_groups + 4 * per_warp - 1) / (4 * per_warp), 128, 0, s>>>(
+                A, tapes, n_leaf_groups, per_warp);
+            ++n_launch;
+        }
         groups_kernel<<<grid, 32 * wpb, group_bytes, s>>>(A, n_leaf_groups);
         if (!cuda_ok(cudaGetLastError(), "leaf kernel")) return LFB_E_CUDA;
         A.smem_regs = qef_regs;
@@ -3843,7 +3864,9 @@ int render_dc_mesh(GpuTape& g, const libfive_region3& R, double min_feature,
         }
         ws.bufs.clear();
         clear_error();
+        ws.lean = true;
         rc = render_in(ws, g, R, min_feature, max_err, out, stats, cancel);
+        ws.lean = false;
     }
     return rc;
 }
@@ -3931,6 +3954,7 @@ int render_dc_meshes(MeshJob* jobs, size_t n, unsigned workers)
         }
         Workspace* w = stream_workspace(0);
         std::lock_guard<std::mutex> lock(w->mu);
+        w->lean = true;
         for (size_t i : retry) {
             MeshJob& j = jobs[i];
             clear_error();
@@ -3939,6 +3963,7 @@ int render_dc_meshes(MeshJob* jobs, size_t n, unsigned workers)
                              j.want_stats ? &j.stats : nullptr, j.cancel);
             if (j.rc != 0) last_error(&j.err);
         }
+        w->lean = false;
     }
 
     clear_error();
