@@ -11,7 +11,7 @@
 #include <functional>
 #include <mutex>
 #include <string>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -943,8 +943,8 @@ void build_ckpt(GpuTape& g)
     for (size_t i = 1; i < jobs.size(); ++i) {
         try {
             other[i] = std::thread(compile, std::ref(jobs[i]));
-        } catch (const std::system_error&) {
-            compile(jobs[i]);   // no thread to be had: here
+        } catch (const std::exception&) {
+            compile(jobs[i]);   // no thread, or no memory for one: here
         }
     }
     if (!jobs.empty()) compile(jobs[0]);

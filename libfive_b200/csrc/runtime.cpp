@@ -4,7 +4,7 @@
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <map>
 
@@ -364,16 +364,18 @@ void host_copy(void* dst, const void* src, size_t bytes)
             std::memcpy(static_cast<char*>(dst) + lo, static_cast<const char*>(src) + lo, hi - lo);
         }
     };
-    std::vector<std::thread> pool;
+    std::thread pool[8];
     for (size_t t = 1; t < n_threads; ++t) {
         try {
-            pool.emplace_back(copy, t);
-        } catch (const std::system_error&) {
-            copy(t);   // no thread to be had: here
+            pool[t] = std::thread(copy, t);
+        } catch (const std::exception&) {
+            copy(t);   // no thread, or no memory for one: here
         }
     }
     copy(0);
-    for (auto& th : pool) th.join();
+    for (auto& th : pool) {
+        if (th.joinable()) th.join();
+    }
 }
 
 }  // namespace lfb
