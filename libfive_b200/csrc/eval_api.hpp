@@ -65,11 +65,12 @@ int eval_grad_with(GpuTape& g, uint64_t n, const float* x, const float* y, const
                    float* gvars, float* scratch, cudaStream_t s);
 
 /// Builds what the reverse mode needs for this tape (partial-slot table,
-/// compiled partials and backward kernels) without launching anything, so
-/// that many tapes can be prepared on several host threads at once.
-bool grad_prepare(GpuTape& g);
-/// True once grad_prepare (or a gradient call) has run for the tape.
-bool grad_prepared(GpuTape& g);
+/// compiled partials and backward kernels, for calls with `points` points)
+/// without launching anything, so that many tapes can be prepared on several
+/// host threads at once.
+bool grad_prepare(GpuTape& g, uint64_t points);
+/// True once grad_prepare (or a gradient call) has run for such calls.
+bool grad_prepared(GpuTape& g, uint64_t points);
 
 /// lfb_fit_adam_step (fit.cu); every pointer as documented there.
 int fit_adam_step(GpuTape* const* tapes, uint32_t n_shapes, const uint64_t* point_offsets,

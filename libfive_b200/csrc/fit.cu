@@ -139,14 +139,11 @@ FitScratch& fit_scratch()
 /// Prepares the reverse mode of every tape that has not been prepared, on
 /// up to 16 host threads (the compiled kernels of a tape are built with
 /// NVRTC, which takes most of a first call).
-int prepare_all(GpuTape* const* tapes, uint32_t n)
+int prepare_all(GpuTape* const* tapes, const uint64_t* poff, uint32_t n)
 {
-    std::vector<GpuTape*> todo;
-    for (uint32_t j = 0; j < n; ++j) {
-        if (!grad_prepared(*tapes[j]) &&
-            std::find(todo.begin(), todo.end(), tapes[j]) == todo.end()) {
-            todo.push_back(tapes[j]);
-        }
+    std::vector<uint32_t> todo;
+    for (uint32_t j = 0; j < n; ++j) {   // no tape is listed twice
+        if (!grad_prepared(*tapes[j], poff[j + 1] - poff[j])) todo.push_back(j);
     }
     if (todo.empty()) return 0;
     int dev = 0;
@@ -166,7 +163,8 @@ int prepare_all(GpuTape* const* tapes, uint32_t n)
             return;
         }
         for (size_t i; (i = next.fetch_add(1)) < todo.size();) {
-            if (!grad_prepare(*todo[i])) {
+            const uint32_t j = todo[i];
+            if (!grad_prepare(*tapes[j], poff[j + 1] - poff[j])) {
                 std::string msg;
                 const int code = last_error(&msg);
                 std::lock_guard<std::mutex> lock(err_mu);
@@ -237,7 +235,7 @@ int fit_adam_step(GpuTape* const* tapes, uint32_t n_shapes, const uint64_t* poff
 
     FitScratch& sc = fit_scratch();
     std::lock_guard<std::mutex> lock(sc.mu);
-    if (int rc = prepare_all(tapes, n_shapes)) return rc;
+    if (int rc = prepare_all(tapes, poff, n_shapes)) return rc;
     if (!sc.f.reserve(n_points * sizeof(float)) ||
         !sc.grad.reserve(std::max<uint64_t>(n_vars, 1) * sizeof(float))) {
         return LFB_E_CUDA;

@@ -464,7 +464,7 @@ int grad_device(GpuTape& g, uint64_t n, const float* x, const float* y, const fl
     // Checkpointed reverse mode when the tape compiles: per point it stores
     // only the registers each tape segment reads from earlier segments, and
     // the backward kernel recomputes the segment from them (jit.cpp).
-    if (const uint32_t ckf = jit_ckpt_prepare(g)) {
+    if (const uint32_t ckf = jit_ckpt_prepare(g, n)) {
         const uint64_t per_point = 4ull * ckf;
         const uint64_t cchunk = std::max<uint64_t>(kBlock, std::min<uint64_t>(
             (4ull << 30) / per_point / kBlock * kBlock, uint64_t(1) << 22));
@@ -602,11 +602,11 @@ int eval_jacobian(GpuTape& g, uint64_t n, const float* x, const float* y, const 
     return cuda_ok(cudaStreamSynchronize(s0), "sync") ? 0 : LFB_E_CUDA;
 }
 
-bool grad_prepare(GpuTape& g)
+bool grad_prepare(GpuTape& g, uint64_t points)
 {
     // the checkpointed kernels, which grad_device takes when they compile;
     // else the stored-partials kernels (m = 0: compile, no launch)
-    if (jit_ckpt_prepare(g)) return true;
+    if (jit_ckpt_prepare(g, points, true)) return true;
     if (!ensure_pslots(g)) return false;
     const uint32_t* hs = g.h_pslot.data();
     jit_partials(g, hs, 0, nullptr, nullptr, nullptr, nullptr, nullptr, 0);
@@ -614,11 +614,11 @@ bool grad_prepare(GpuTape& g)
     return true;
 }
 
-bool grad_prepared(GpuTape& g)
+bool grad_prepared(GpuTape& g, uint64_t points)
 {
+    if (jit_ckpt_ready(g, points)) return true;
     std::lock_guard<std::mutex> lock(g.mu);
-    if (g.jit[5].state == 1 && g.jit[6].state == 1) return true;
-    return g.jit[5].state != 0 && g.jit[6].state != 0 && g.pslot_ready &&
+    return g.jit[5].state != 0 && (g.jit[6].state != 0 || g.jit[7].state != 0) && g.pslot_ready &&
            g.jit[2].state != 0 && g.jit[3].state != 0;
 }
 
@@ -672,7 +672,7 @@ int eval_loss_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const
     auto& st = grad_staging();
     if (!st.out.reserve(sizeof(double))) return LFB_E_CUDA;
     double* sum = st.out.as<double>();
-    if (const uint32_t ckf = jit_ckpt_prepare(g)) {
+    if (const uint32_t ckf = jit_ckpt_prepare(g, n)) {
         // one forward pass gives f and the checkpoints; the backward pass
         // takes seed 2 f_i / n
         const uint64_t per_point = 4ull * ckf;
@@ -721,7 +721,7 @@ int eval_loss_grad(GpuTape& g, uint64_t n, const float* x, const float* y, const
 
 uint64_t grad_scratch_floats(GpuTape& g, uint64_t n)
 {
-    const uint32_t ckf = tape_has_const_var(g) ? 0 : jit_ckpt_prepare(g);
+    const uint32_t ckf = tape_has_const_var(g) ? 0 : jit_ckpt_prepare(g, n, true);
     // one launch pair: no more points than grad_device takes at once
     return ckf && n <= (uint64_t(1) << 22) ? n * ckf : 0;
 }

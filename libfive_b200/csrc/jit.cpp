@@ -915,10 +915,10 @@ bool build(GpuTape& g, int k, const std::string& src, const char* name)
 /// (ckpt_three).
 bool has_ckpt_three(const GpuTape& g) { return g.reg.clauses.size() > 2 * kJitSegClauses; }
 
-/// Compiles the checkpointed reverse mode's kernels that the tape has, each
-/// on a thread of its own, so that a later call never waits for a compiler
-/// whatever its number of points.  With g.mu held.
-void build_ckpt(GpuTape& g)
+/// Compiles the checkpointed reverse mode's kernels, forward and backward
+/// (bit k of `want`: slot k), those that the tape has not, each on a thread of
+/// its own.  With g.mu held.
+void build_ckpt(GpuTape& g, uint32_t want)
 {
     struct Job {
         int k;
@@ -928,8 +928,8 @@ void build_ckpt(GpuTape& g)
     };
     std::vector<Job> jobs;
     const bool fits = api().ok && g.reg.clauses.size() <= kJitMaxSegmentedClauses;
-    for (int k = 5; k <= (has_ckpt_three(g) ? 7 : 6); ++k) {
-        if (g.jit[k].state) continue;
+    for (int k = 5; k <= 7; ++k) {
+        if (g.jit[k].state || !(want >> k & 1)) continue;
         g.jit[k].state = -1;
         if (fits) jobs.push_back({k, k == 5 ? ckpt_forward_source(g.reg) : ckpt_backward_source(g.reg, k == 7), {}, false});
     }
@@ -962,7 +962,7 @@ void* kernel(GpuTape& g, int k, const std::vector<uint32_t>* slots = nullptr)
     std::lock_guard<std::mutex> lock(g.mu);
     GpuTape::JitKernel& j = g.jit[k];
     if (j.state == 0 && k >= 5) {
-        build_ckpt(g);
+        build_ckpt(g, 1u << k);
     } else if (j.state == 0) {
         const size_t n = g.reg.clauses.size();
         bool ok = api().ok && n <= (k == 4 ? kJitMaxIntervalClauses
@@ -1108,10 +1108,24 @@ bool jit_ckpt_fills_gpu(const GpuTape& g, uint64_t points)
     return g.reg.clauses.size() > 8 * kJitSegClauses && 2 * points > wave && points <= wave;
 }
 
-uint32_t jit_ckpt_prepare(GpuTape& g)
+bool jit_ckpt_ready(GpuTape& g, uint64_t points)
 {
-    if (!kernel(g, 5) || !kernel(g, 6)) return 0;
     std::lock_guard<std::mutex> lock(g.mu);
+    return g.jit[5].state == 1 && g.jit[ckpt_three(g, points) ? 7 : 6].state == 1;
+}
+
+uint32_t jit_ckpt_prepare(GpuTape& g, uint64_t points, bool only_these)
+{
+    std::lock_guard<std::mutex> lock(g.mu);
+    const int k = ckpt_three(g, points) ? 7 : 6;
+    if (g.jit[k].state == 0) {
+        const bool all = g.jit[5].state == 0 && !only_these && has_ckpt_three(g);
+        build_ckpt(g, 1u << 5 | 1u << k | (all ? 3u << 6 : 0u));
+    }
+    if (g.jit[k].state != 1 && g.jit[13 - k].state == 0 && has_ckpt_three(g)) {
+        build_ckpt(g, 1u << (13 - k));   // the other one
+    }
+    if (g.jit[5].state != 1 || (g.jit[6].state != 1 && g.jit[7].state != 1)) return 0;
     if (!g.ckpt_floats) {
         uint32_t total = 0;
         jit_segments(g.reg, &total);
@@ -1138,8 +1152,15 @@ bool jit_ckpt_backward(GpuTape& g, uint32_t m, const float* C, const float* seed
     uint32_t n_vars = g.reg.n_vars;
     const unsigned smem = gvars ? n_vars * 4 : 0;
     if (smem > 48 * 1024) return false;
-    void* fn = ckpt_three(g, m) ? kernel(g, 7) : nullptr;
-    if (!fn) fn = kernel(g, 6);
+    // the form for this many points, or the one that there is
+    void* fn = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g.mu);
+        const int k = ckpt_three(g, m) ? 7 : 6;
+        for (int i : {k, 13 - k}) {
+            if (!fn && g.jit[i].state == 1) fn = g.jit[i].function;
+        }
+    }
     if (!fn) return false;
     if (m == 0) return true;
     const float* cp = g.d_cpool;

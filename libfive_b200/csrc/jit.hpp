@@ -78,11 +78,16 @@ bool jit_compile(const std::string& src, std::vector<char>* cubin, std::string* 
 /// segments (C[slot * m + i], jit_ckpt_prepare's count of slots); the
 /// backward kernel recomputes each segment from them and sweeps its
 /// adjoints back, with the products and sums of the partials / backward
-/// kernels.  jit_ckpt_prepare compiles both (the backward kernel of longer
-/// tapes in two forms, of which each call takes the one for its number of
-/// points) and returns the slot count, or 0 when the tape has no compiled
-/// form.
-uint32_t jit_ckpt_prepare(GpuTape& g);
+/// kernels.  The backward kernel of longer tapes has two forms, of which each
+/// call takes the one for its number of points.  jit_ckpt_prepare compiles
+/// what a call with `points` points needs, a tape's first call both forms
+/// beside each other, so that a later call of another size waits for no
+/// compiler; only_these: this call's form alone (many tapes prepared at once
+/// share the processors).  It returns the slot count, or 0 when the tape has
+/// no compiled form.
+uint32_t jit_ckpt_prepare(GpuTape& g, uint64_t points, bool only_these = false);
+/// Whether jit_ckpt_prepare has nothing left to compile for such a call.
+bool jit_ckpt_ready(GpuTape& g, uint64_t points);
 /// Whether `points` points of a long tape keep the GPU busy by themselves: one
 /// wave of the backward kernel that is more than half full, with code that
 /// fills the instruction cache.

@@ -5,8 +5,10 @@ import time
 
 import numpy as np
 import pytest
+import torch
 
 from libfive_b200 import workloads
+from libfive_b200.fit import BatchedFit
 from libfive_b200.shape import Tape
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +41,17 @@ def test_any_order(gpu, order):
         for a, b in zip(got, want):
             assert np.array_equal(a, b, equal_nan=True)
         assert np.isfinite(gvars).all()
+
+
+def test_after_a_fit(gpu):
+    """A fit step compiles the form for its own points; a call that wants the
+    other one gets it."""
+    shape, vals, _ = workloads.fit_csg_vars(48, seed=79)
+    tape = Tape(shape, vals)
+    points = [tuple(torch.from_numpy(a).cuda() for a in workloads.uniform_points(1000, seed=5))]
+    BatchedFit([tape], points, lr=0.0).step()
+    for n in (120001, 50000):
+        _, got, _ = gradient(tape, n)
+        _, want, _ = gradient(Tape(shape, vals), n)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b, equal_nan=True)
