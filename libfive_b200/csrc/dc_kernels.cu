@@ -94,12 +94,12 @@ __device__ __forceinline__ WideConsts wide_consts(const uint4& e, const float* _
 
 /// Interval of list entry k, stored in slot 3 + k, and the entry's state for
 /// the cell's children; returns whether a min/max got decided
-/// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167); enclosing:
+/// (IntervalEvaluator::eval + push, eval_interval.cpp:116-167); ENCLOSING:
 /// intervals enclose what the point interpreters compute, and nothing is
 /// decided between operands that may be NaN.
+template <bool ENCLOSING = false>
 __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c, uint32_t k,
-                                             float2* S, uint8_t* SN, uint8_t* pst,
-                                             bool enclosing = false)
+                                             float2* S, uint8_t* SN, uint8_t* pst)
 {
     const uint8_t o = e.x & 0xff;
     const uint32_t kinds = (e.x >> 8) & 0xf;
@@ -119,11 +119,11 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
             uint8_t keep = 0;   // 0 both, 1 a, 2 b
             if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;
             else if (b.lo > a.hi) keep = (o == op::MAX) ? 2 : 1;
-            if (keep && !(enclosing && (a.nan || b.nan))) {
+            if (keep && !(ENCLOSING && (a.nan || b.nan))) {
                 ps = keep == 1 ? WIDE_A : WIDE_B;
                 decided = true;
             }
-        } else if (enclosing) {
+        } else if (ENCLOSING) {
             r = iv_enclose(o, a, b, r);
         }
     }
@@ -563,7 +563,14 @@ __device__ __forceinline__ uint32_t warp_counts_scan(uint32_t count, uint32_t* w
     return __shfl_sync(0xffffffffu, incl - v, warp);
 }
 
-__global__ void __launch_bounds__(kBlockThreads, 2)
+/// boxes: the box form (WideArgs::boxes) is an instance of its own, so that
+/// the levels' form carries nothing of it.  per_sm: blocks that share an SM;
+/// where a list's state leaves room for one only, that one has 128 registers
+/// a thread instead of 64, which spill in the box form (derivatives of a
+/// 1,500-primitive CSG at 100,003 points 2.10 -> 1.90 ms, of a union of 1,200
+/// spheres 3.01 -> 2.67 ms).
+template <bool boxes, int per_sm>
+__global__ void __launch_bounds__(kBlockThreads, per_sm)
 k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
 {
     extern __shared__ __align__(16) unsigned char bsm[];
@@ -575,7 +582,6 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
     const Octree& o = A.o;
     const LevelView& lv = o.lv[d];
     const DevTape& bt = A.bt;
-    const bool boxes = A.boxes != nullptr;
     const uint32_t n_cells = boxes ? A.n_boxes : lv.n_cells;
     const uint32_t n = A.n;
     const size_t slot = blockIdx.x;
@@ -655,7 +661,7 @@ k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)
             fetch(w + 1, e_next);
             c_next = wide_consts(e_next, bt.cpool);
             for (uint32_t l = lf; l <= ll; ++l) {
-                if (lev == l) changed |= wide_forward(e, c, k, S, SN, pst, boxes);
+                if (lev == l) changed |= wide_forward<boxes>(e, c, k, S, SN, pst);
                 __syncthreads();
             }
             e = e_next;
@@ -2825,12 +2831,14 @@ uint32_t interval_box_slots(uint32_t n, uint32_t n_boxes)
 
 cudaError_t launch_interval_boxes(const WideArgs& W, uint32_t slots, cudaStream_t s)
 {
-    const uint32_t n_slots = block_slots(W.n, block_slots(W.n, 2) >= W.n ? 2 : 1);
+    const uint32_t per_sm = block_slots(W.n, 2) >= W.n ? 2 : 1;
+    const uint32_t n_slots = block_slots(W.n, per_sm);
     const size_t smem = block_smem(n_slots);
-    if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_block), smem)) {
+    auto* kernel = per_sm == 2 ? k_interval_block<true, 2> : k_interval_block<true, 1>;
+    if (!raise_smem_limit(reinterpret_cast<const void*>(kernel), smem)) {
         return cudaErrorInvalidValue;
     }
-    k_interval_block<<<std::max<uint32_t>(slots, 1), kBlockThreads, smem, s>>>(W, 0, n_slots);
+    kernel<<<std::max<uint32_t>(slots, 1), kBlockThreads, smem, s>>>(W, 0, n_slots);
     return cudaGetLastError();
 }
 
@@ -2845,12 +2853,12 @@ cudaError_t launch_interval_lists(const WideArgs& W, int d, uint32_t n_cells, ui
         const uint32_t per_sm = n_cells <= sms ? 1 : 2;
         const uint32_t slots = block_slots(W.n, per_sm);
         const size_t smem = block_smem(slots);
-        if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_block), smem)) {
+        if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_block<false, 2>), smem)) {
             return cudaErrorInvalidValue;
         }
         const uint32_t blocks = std::min<uint32_t>(std::min<uint32_t>(scratch_warps, sms * per_sm),
                                                    n_cells);
-        k_interval_block<<<std::max<uint32_t>(blocks, 1), kBlockThreads, smem, s>>>(W, d, slots);
+        k_interval_block<false, 2><<<std::max<uint32_t>(blocks, 1), kBlockThreads, smem, s>>>(W, d, slots);
     } else {
         const size_t smem = sizeof(WideSmem) * 8;
         if (!raise_smem_limit(reinterpret_cast<const void*>(k_interval_wide), smem)) {

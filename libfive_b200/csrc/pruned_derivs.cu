@@ -15,13 +15,15 @@
 //      when its operands' intervals are disjoint and neither may be NaN, so
 //      that at every point of the cell the kept operand is the one that the
 //      full tape takes, value and partials alike;
-//   3. one block per cell runs the derivative interpreter over its own tape.
+//   3. a warp for every 32 points of a cell runs the derivative interpreter
+//      over the cell's tape, the warps of the longest tapes first.
 //
 // Results are the full tape's, bit for bit.  Nothing here waits for the
 // device: a pruned tape that does not fit the arena is replaced by the full
 // one, and scratch is allocated and freed in stream order.
-// 100,003 points over an 18,900-clause CSG tape: 7.08 -> 2.25 ms (sorting 0.08,
-// intervals 0.68, the interpreter 1.45).
+// 100,003 points over an 18,900-clause CSG tape: 1.99 ms (the whole tape 9.26;
+// sorting 0.08, intervals 0.69, the interpreter most of the rest); 256 points
+// 2.72 ms (3.31), 10^6 points 6.98 ms (78.5).
 #include <cub/cub.cuh>
 
 #include <algorithm>
