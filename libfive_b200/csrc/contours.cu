@@ -1039,6 +1039,7 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
     // kMaxTapeRegs registers, dependency chains too long for a list) start
     // with a thread a cell.
     constexpr uint32_t kListCells = 8192;
+    constexpr int kListDepth = 21;   // deepest whose cells' indices fit pack_coords
     const bool lists_ok = bt.n && bt.n_regs <= kMaxTapeRegs && g.ensure_wide();
     if (!lists_ok) clear_error();
 
@@ -1185,7 +1186,7 @@ int render_contours(GpuTape& g, const double lo[2], const double hi[2], double z
             cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flags, scan, n + 1, s);
             void* tmp = B.get<unsigned char>(CB::SCANTMP, tmp_bytes);
             if (!out_tape || !flags || !scan || !tmp) return LFB_E_CUDA;
-            lists = lists && n < kListCells;
+            lists = lists && n < kListCells && d <= kListDepth;
             ListRef* cell_list = nullptr;
             uint32_t n_branch = 0;
             for (int again = 0;; ++again) {
