@@ -114,7 +114,7 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
     } else {
         const Iv a = wide_fetch(kinds & 3, e.y, c.a, S, SN);
         const Iv b = dev_is_binary(o) ? wide_fetch((kinds >> 2) & 3, e.z, c.b, S, SN) : a;
-        r = iv_eval(o, a, b);
+        r = iv_eval<ENCLOSING>(o, a, b);
         if (o == op::MIN || o == op::MAX) {
             uint8_t keep = 0;   // 0 both, 1 a, 2 b
             if (a.lo > b.hi) keep = (o == op::MAX) ? 1 : 2;
@@ -123,8 +123,6 @@ __device__ __forceinline__ bool wide_forward(const uint4& e, const WideConsts& c
                 ps = keep == 1 ? WIDE_A : WIDE_B;
                 decided = true;
             }
-        } else if (ENCLOSING) {
-            r = iv_enclose(o, a, b, r);
         }
     }
     S[3 + k] = make_float2(r.lo, r.hi);
@@ -567,8 +565,8 @@ __device__ __forceinline__ uint32_t warp_counts_scan(uint32_t count, uint32_t* w
 /// the levels' form carries nothing of it.  per_sm: blocks that share an SM;
 /// where a list's state leaves room for one only, that one has 128 registers
 /// a thread instead of 64, which spill in the box form (derivatives of a
-/// 1,500-primitive CSG at 100,003 points 2.10 -> 1.90 ms, of a union of 1,200
-/// spheres 3.01 -> 2.67 ms).
+/// 1,500-primitive CSG at 100,003 points 2.10 -> 1.92 ms, of a union of 1,200
+/// spheres 3.01 -> 2.66 ms).
 template <bool boxes, int per_sm>
 __global__ void __launch_bounds__(kBlockThreads, per_sm)
 k_interval_block(const __grid_constant__ WideArgs A, int d, uint32_t smem_slots)

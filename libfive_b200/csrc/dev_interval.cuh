@@ -463,39 +463,12 @@ __device__ __forceinline__ Iv iv_apply(uint8_t o, const Iv& a, const Iv& b)
     return dev_is_binary(o) ? iv_binary(o, a, b) : iv_unary(o, a);
 }
 
-/// The operations with long bodies, out of line and by value (operands and
-/// result stay in registers).
-static __device__ __noinline__ Iv iv_rare(uint8_t o, Iv a, Iv b)
-{
-    return iv_apply(o, a, b);
-}
-
-/// iv_apply for the tape interpreters: the frequent operations inline, each
-/// its own case, the others in a call.  (With all of them inline the
-/// dispatch was a call through local memory per clause.)
-__device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
-{
-    switch (o) {
-        case op::ADD: return iv_binary(op::ADD, a, b);
-        case op::SUB: return iv_binary(op::SUB, a, b);
-        case op::MUL: return iv_binary(op::MUL, a, b);
-        case op::MIN: return iv_binary(op::MIN, a, b);
-        case op::MAX: return iv_binary(op::MAX, a, b);
-        case op::SQUARE: return iv_unary(op::SQUARE, a);
-        case op::SQRT: return iv_unary(op::SQRT, a);
-        case op::NEG: return iv_unary(op::NEG, a);
-        case op::ABS: return iv_unary(op::ABS, a);
-        case OP_COPY: return a;
-        default: return iv_rare(o, a, b);
-    }
-}
-
 __device__ __forceinline__ Iv iv_not_empty(const Iv& a)
 {
     return iv_bad(a) ? Iv{-LF_INF, LF_INF, true} : a;
 }
 
-/// r = iv_eval(o, a, b) made an enclosure of every value that the point
+/// r = iv_apply(o, a, b) made an enclosure of every value that the point
 /// interpreters compute for operands in a and b.  The rules above are the
 /// reference's, which a mesh needs to be its mesh; where they leave values
 /// out, a min / max decided by them can drop the operand that a point takes:
@@ -513,6 +486,42 @@ __device__ __forceinline__ Iv iv_enclose(uint8_t o, const Iv& a, const Iv& b, Iv
     if (o == op::SUB && a.hi == LF_INF && b.hi == LF_INF) r.nan = true;
     if (o == op::RECIP && a.lo <= 0.0f && a.hi >= 0.0f) r = {-LF_INF, LF_INF, a.nan};
     return iv_not_empty(r);
+}
+
+/// The operations with long bodies, out of line and by value (operands and
+/// result stay in registers).
+template <bool ENCLOSING>
+static __device__ __noinline__ Iv iv_rare(uint8_t o, Iv a, Iv b)
+{
+    const Iv r = iv_apply(o, a, b);
+    return ENCLOSING ? iv_enclose(o, a, b, r) : r;
+}
+
+/// iv_apply for the tape interpreters: the frequent operations inline, each
+/// its own case, the others in a call.  (With all of them inline the
+/// dispatch was a call through local memory per clause.)  ENCLOSING: with
+/// iv_enclose's corrections, in each case its own.
+template <bool ENCLOSING = false>
+__device__ __forceinline__ Iv iv_eval(uint8_t o, const Iv& a, const Iv& b)
+{
+    Iv r;
+    switch (o) {
+        case op::ADD: r = iv_binary(op::ADD, a, b); break;
+        case op::SUB:
+            r = iv_binary(op::SUB, a, b);
+            if (ENCLOSING) r = iv_enclose(op::SUB, a, b, r);
+            return r;
+        case op::MUL: r = iv_binary(op::MUL, a, b); break;
+        case op::MIN: return iv_binary(op::MIN, a, b);
+        case op::MAX: return iv_binary(op::MAX, a, b);
+        case op::SQUARE: r = iv_unary(op::SQUARE, a); break;
+        case op::SQRT: r = iv_unary(op::SQRT, a); break;
+        case op::NEG: r = iv_unary(op::NEG, a); break;
+        case op::ABS: r = iv_unary(op::ABS, a); break;
+        case OP_COPY: return a;
+        default: return iv_rare<ENCLOSING>(o, a, b);
+    }
+    return ENCLOSING ? iv_not_empty(r) : r;
 }
 
 /// Interval::state(): AMBIGUOUS when the value may be NaN.

@@ -21,9 +21,9 @@
 // Results are the full tape's, bit for bit.  Nothing here waits for the
 // device: a pruned tape that does not fit the arena is replaced by the full
 // one, and scratch is allocated and freed in stream order.
-// 100,003 points over an 18,900-clause CSG tape: 1.99 ms (the whole tape 9.26;
-// sorting 0.08, intervals 0.69, the interpreter most of the rest); 256 points
-// 2.72 ms (3.31), 10^6 points 6.98 ms (78.5).
+// 100,003 points over an 18,667-clause CSG tape: 1.92 ms (the whole tape
+// 11.2; sorting 0.08, intervals 0.58, the interpreter 1.23); 256 points 2.70 ms
+// (3.31), 10^6 points 6.86 ms (78.5).
 #include <cub/cub.cuh>
 
 #include <algorithm>
