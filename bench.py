@@ -419,10 +419,9 @@ def run_ours(args, world, rank, local):
                 "clause_evals_per_launch": (evals_v + evals_g) / args.steps,
                 "kernel_ms_per_launch": leaf_ms / args.steps,
                 "traffic": traffic,
-                "traffic_source": ("ncu capture of the leaf stage's four kernels on this "
+                "traffic_source": ("ncu capture of the leaf stage's kernels on this "
                                    "workload, dram__bytes_read.sum + dram__bytes_write.sum "
-                                   "(profiles/k_leaf_groups_csg2000_depth10_dram.md), taken "
-                                   "before the leaf stage ran in fused steps"
+                                   "(profiles/k_leaf_groups_csg2000_depth10_dram.md)"
                                    if traffic is not None else None),
             },
             "stages_ms": {"interval": stats.ms_interval, "leaf": stats.ms_leaf,
