@@ -262,8 +262,9 @@ int lfb_render_meshes(const lfb_tape* tapes, uint32_t n,
  *        as if cudaMalloc had run out of memory (the call in progress fails
  *        with LFB_E_CUDA; nothing else is affected);
  *    "small_capacity" 1: every mesh starts from empty scratch buffers and
- *        minimal tape-arena, list and dual-walk capacities, so each growth
- *        and retry path runs.
+ *        minimal tape-arena, list and dual-walk capacities, and every slice
+ *        from minimal arena, list, record and segment capacities, so each
+ *        growth and retry path runs.
  *  Returns 0, or LFB_E_INVALID for an unknown key. */
 int lfb_debug_set(const char* key, int64_t value);
 

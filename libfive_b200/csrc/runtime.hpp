@@ -115,8 +115,8 @@ std::shared_ptr<GpuTape> cached_tape(const Node* root);
 void invalidate_cached(const Node* root);
 
 /// Test hooks (lfb_debug_set): the number of device allocations left before
-/// one is made to fail (0: none is), and whether meshes start from minimal
-/// capacities.
+/// one is made to fail (0: none is), and whether meshes and slices start from
+/// minimal capacities.
 struct DebugHooks {
     std::atomic<int64_t> fail_alloc_after{0};
     std::atomic<int> small_capacity{0};
